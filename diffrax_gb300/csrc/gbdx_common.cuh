@@ -515,6 +515,7 @@ struct SolveParams {
   uint64_t seed;              // Brownian generator seed
   double vbt_t0, vbt_len, vbt_tol_unit;
   double vbt_inv_len;         // 1 / vbt_len
+  int vbt_levels;             // least level with 2^-level <= vbt_tol_unit (in FP32)
   float vbt_sqrt_len;         // sqrt(vbt_len) as FP32
   // Recursive-checkpoint tape (forward pass of a differentiated solve)
   double *tape_t;             // [batch, max_steps + 1] accepted-step time grid

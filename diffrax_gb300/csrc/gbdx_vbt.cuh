@@ -13,6 +13,7 @@
 #include <stdint.h>
 
 #include "gbdx_common.cuh"
+#include "gbdx_f2.cuh"
 
 namespace gbdx {
 
@@ -33,183 +34,245 @@ __device__ __forceinline__ void philox4x32_10(uint32_t (&c)[4], uint32_t k0, uin
 
 enum { kVbtRoot = 0, kVbtMid = 1, kVbtLeaf = 2, kVbtRootH = 3, kVbtMidH = 4, kVbtLeafH = 5 };
 
+// Two Box--Muller pairs from 24-bit uniforms: u = ((ua >> 8) + 1/2) 2^-24 and v
+// alike give (sqrt(-2 log u) cos 2 pi v, sqrt(-2 log u) sin 2 pi v) in z[0], z[1];
+// ub, vb in z[2], z[3].  A draw costs as much as the rest of the descent, so the
+// functions are spelled out on the packed FP32x2 pipe: log as e ln 2 + log1p(f), u
+// = (1 + f) 2^e with 1 + f in [sqrt 1/2, sqrt 2) and a minimax fit (6e-9 relative);
+// cos and sin of pi/2 r, r the distance of 4 v from its quadrant (fits 3e-9, 5e-11
+// relative; v needs no other reduction).  Each value is within about two units in
+// the last place, as logf, sqrtf and sincospif give it, at a third of their issue
+// slots.
+__device__ __forceinline__ void box_muller2(uint32_t ua, uint32_t va, uint32_t ub, uint32_t vb,
+                                            float (&z)[4]) {
+  // (k + 1/2) 2^-24 = (2 k + 1) 2^-25, one rounding
+  const F2 u = f2_mul(f2_pack(float((ua >> 7) | 1u), float((ub >> 7) | 1u)),
+                      f2_set(0x1p-25f));
+  const F2 q = f2_mul(f2_pack(float((va >> 7) | 1u), float((vb >> 7) | 1u)),
+                      f2_set(0x1p-23f));  // 4 v
+  float u0, u1;
+  f2_unpack(u, u0, u1);
+  const int i0 = __float_as_int(u0), i1 = __float_as_int(u1);
+  const int e0 = (i0 - 0x3f3504f3) >> 23, e1 = (i1 - 0x3f3504f3) >> 23;
+  const F2 f = f2_add(f2_pack(__int_as_float(i0 - (e0 << 23)), __int_as_float(i1 - (e1 << 23))),
+                      f2_set(-1.f));
+  // the exponents as floats (1.5 2^23 + e is exact)
+  const F2 e = f2_add(f2_pack(__int_as_float(0x4b400000 + e0), __int_as_float(0x4b400000 + e1)),
+                      f2_set(-12582912.f));
+  F2 p = f2_set(-0.07634474337100983f);
+  p = f2_fma(p, f, f2_set(0.12761567533016205f));
+  p = f2_fma(p, f, f2_set(-0.13160187005996704f));
+  p = f2_fma(p, f, f2_set(0.14201758801937103f));
+  p = f2_fma(p, f, f2_set(-0.16623356938362122f));
+  p = f2_fma(p, f, f2_set(0.20001226663589478f));
+  p = f2_fma(p, f, f2_set(-0.2500081956386566f));
+  p = f2_fma(p, f, f2_set(0.3333333134651184f));
+  p = f2_fma(p, f, f2_set(-0.5f));
+  const F2 lg = f2_fma(e, f2_set(0.6931471824645996f), f2_fma(f2_mul(f, f), p, f));
+  float l0, l1, r0, r1;
+  f2_unpack(f2_mul(lg, f2_set(-2.f)), l0, l1);
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(l0));
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r1) : "f"(l1));
+  // quadrant and distance
+  const F2 big = f2_add(q, f2_set(12582912.f));
+  float b0, b1;
+  f2_unpack(big, b0, b1);
+  const int n0 = __float_as_int(b0), n1 = __float_as_int(b1);
+  const F2 r = f2_fma(f2_add(big, f2_set(-12582912.f)), f2_set(-1.f), q), w = f2_mul(r, r);
+  F2 s = f2_set(-0.004601656924933195f);
+  s = f2_fma(s, w, f2_set(0.07968003302812576f));
+  s = f2_fma(s, w, f2_set(-0.6459634304046631f));
+  s = f2_mul(f2_fma(s, w, f2_set(1.5707963705062866f)), r);
+  F2 c = f2_set(0.0009040216682478786f);
+  c = f2_fma(c, w, f2_set(-0.02086028829216957f));
+  c = f2_fma(c, w, f2_set(0.25366923213005066f));
+  c = f2_fma(c, w, f2_set(-1.2337005138397217f));
+  c = f2_fma(c, w, f2_set(1.f));
+  float s0, s1, c0, c1;
+  f2_unpack(f2_mul(s, f2_pack(r0, r1)), s0, s1);
+  f2_unpack(f2_mul(c, f2_pack(r0, r1)), c0, c1);
+  // cos: c, -s, -c, s; sin: s, c, -s, -c for quadrants 0..3
+  auto turn = [](float x, int n) {
+    return __int_as_float(__float_as_int(x) ^ ((n & 2) << 30));
+  };
+  z[0] = turn(n0 & 1 ? s0 : c0, n0 + 1);
+  z[1] = turn(n0 & 1 ? c0 : s0, n0);
+  z[2] = turn(n1 & 1 ? s1 : c1, n1 + 1);
+  z[3] = turn(n1 & 1 ? c1 : s1, n1);
+}
+
+__device__ __forceinline__ void vbt_philox(uint64_t seed, uint32_t traj, uint32_t node,
+                                           uint32_t kind, int quad, uint32_t (&c)[4]) {
+  c[0] = traj;
+  c[1] = node;
+  c[2] = (kind << 24) | uint32_t(quad);
+  c[3] = 0x5EEDu;
+  philox4x32_10(c, uint32_t(seed), uint32_t(seed >> 32));
+}
+
 // Normals of dimensions (col, col + 1), col even, for one tree node.
 __device__ __forceinline__ float2 vbt_normal_pair(uint64_t seed, uint32_t traj, uint32_t node,
                                                   uint32_t kind, int col) {
-  uint32_t c[4] = {traj, node, (kind << 24) | uint32_t(col >> 2), 0x5EEDu};
-  philox4x32_10(c, uint32_t(seed), uint32_t(seed >> 32));
-  const int p = (col >> 1) & 1;  // which Box-Muller pair of the quad
-  const float u = (float(c[2 * p] >> 8) + 0.5f) * (1.0f / 16777216.0f);
-  const float v = (float(c[2 * p + 1] >> 8) + 0.5f) * (1.0f / 16777216.0f);
-  const float rad = sqrtf(-2.0f * logf(u));
-  float s, co;
-  sincospif(2.0f * v, &s, &co);
-  return make_float2(rad * co, rad * s);
+  uint32_t c[4];
+  vbt_philox(seed, traj, node, kind, col >> 2, c);
+  const bool p = col & 2;  // which Box-Muller pair of the quad
+  float z[4];
+  box_muller2(p ? c[2] : c[0], p ? c[3] : c[1], 0u, 0u, z);
+  return make_float2(z[0], z[1]);
 }
 
-// sqrt(T) W_unit(r) for dimensions (col, col + 1) of trajectory `traj` at time t.
-static __device__ __noinline__ float2 vbt_w_pair(const SolveParams &P, int64_t traj, double t,
-                                          int col) {
-  const float r = float((t - P.vbt_t0) * P.vbt_inv_len);
-  const float tol = float(P.vbt_tol_unit);
-  const uint32_t tj = uint32_t(traj);
-  float2 z = vbt_normal_pair(P.seed, tj, 0u, kVbtRoot, col);
-  float ws0 = 0.f, ws1 = 0.f, wsu0 = z.x, wsu1 = z.y;
-  float s = 0.f, su = 1.f;
-  uint32_t node = 1;
-  // while 2^-level > tol (tree.py:406-409)
-  while (su > tol) {
-    const float st = 0.5f * su, t_mid = s + st;
-    z = vbt_normal_pair(P.seed, tj, node, kVbtMid, col);
-    const float a = 0.5f * sqrtf(su);
-    const float m0 = 0.5f * wsu0, m1 = 0.5f * wsu1;
-    const float st0 = m0 + a * z.x, st1 = m1 + a * z.y;  // W_{s,t}
-    const float tu0 = m0 - a * z.x, tu1 = m1 - a * z.y;  // W_{t,u}
-    const bool right = r > t_mid;
-    if (right) {
-      ws0 += st0;
-      ws1 += st1;
-      wsu0 = tu0;
-      wsu1 = tu1;
-      s = t_mid;
-    } else {
-      wsu0 = st0;
-      wsu1 = st1;
-    }
-    node = 2 * node + (right ? 1u : 0u);
-    su = st;
-  }
-  const float sr = fmaxf(r - s, 0.f), ru = fmaxf(su - sr, 0.f);
-  z = vbt_normal_pair(P.seed, tj, node, kVbtLeaf, col);
-  const float bb = sqrtf(sr * ru / su), f = sr / su;
-  const float sq = P.vbt_sqrt_len;
-  return make_float2(sq * (ws0 + f * wsu0 + bb * z.x), sq * (ws1 + f * wsu1 + bb * z.y));
-}
-
-// Normals of the quad of dimensions 4 quad .. 4 quad + 3 for one tree node:
-// both Box-Muller pairs of one Philox block (vbt_normal_pair returns one).
-__device__ __forceinline__ float4 vbt_normal_quad(uint64_t seed, uint32_t traj, uint32_t node,
-                                                  uint32_t kind, int quad) {
-  uint32_t c[4] = {traj, node, (kind << 24) | uint32_t(quad), 0x5EEDu};
-  philox4x32_10(c, uint32_t(seed), uint32_t(seed >> 32));
-  float out[4];
-#pragma unroll
-  for (int p = 0; p < 2; p++) {
-    const float u = (float(c[2 * p] >> 8) + 0.5f) * (1.0f / 16777216.0f);
-    const float v = (float(c[2 * p + 1] >> 8) + 0.5f) * (1.0f / 16777216.0f);
-    const float rad = sqrtf(-2.0f * logf(u));
-    float sn, co;
-    sincospif(2.0f * v, &sn, &co);
-    out[2 * p] = rad * co;
-    out[2 * p + 1] = rad * sn;
-  }
-  return make_float4(out[0], out[1], out[2], out[3]);
-}
-
-// The bridge state of one descent path for a quad of dimensions: W at the
-// start of each level's dyadic interval and the increment across it.
-// Consecutive evaluations of a solve lie close together, so their paths share
-// the upper levels; an evaluation re-descends only below the deepest level
-// whose interval also contains the new time.
-constexpr int kVbtCacheLevels = 24;
-struct VbtQuadCache {
-  float ws[kVbtCacheLevels + 1][4], wsu[kVbtCacheLevels + 1][4];
-  uint32_t node;  // heap index of the cached path's leaf interval
-  long long traj; // trajectory of the cached path (-1: none)
-};
-
-// sqrt(T) W_unit(r) for the quad of dimensions of trajectory `traj` at time t:
-// the values of vbt_w_pair, descending from the cached path.
-static __device__ __noinline__ float4 vbt_w_quad(const SolveParams &P, int64_t traj, double t, int quad,
-                                          VbtQuadCache &C) {
-  const float r = float((t - P.vbt_t0) * P.vbt_inv_len);
-  const float tol = float(P.vbt_tol_unit);
-  const uint32_t tj = uint32_t(traj);
-  // the new path: levels and leaf node, by the comparisons of vbt_w_pair
-  float s = 0.f, su = 1.f;
-  uint32_t node = 1;
-  int L = 0;
-  while (su > tol) {
-    const float st = 0.5f * su, tm = s + st;
-    const bool right = r > tm;
-    if (right) s = tm;
-    node = 2 * node + (right ? 1u : 0u);
-    su = st;
-    L++;
-  }
-  int d = 0;
-  if (L <= kVbtCacheLevels && C.traj == (long long)traj) {
-    const uint32_t x = node ^ C.node;
-    d = x == 0 ? L : L - 1 - (31 - __clz(x));  // levels shared with the cached path
+// Normals of NQ dimensions for two nodes: NQ = 4, a quad's; NQ = 2, those of pair
+// `sel` of the quad.  The two nodes' draws are independent, so they overlap.
+template <int NQ>
+__device__ __forceinline__ void vbt_normals2(uint64_t seed, uint32_t traj, uint32_t node0,
+                                             uint32_t kind0, uint32_t node1, uint32_t kind1,
+                                             int quad, int sel, float (&z0)[NQ],
+                                             float (&z1)[NQ]) {
+  uint32_t a[4], b[4];
+  vbt_philox(seed, traj, node0, kind0, quad, a);
+  vbt_philox(seed, traj, node1, kind1, quad, b);
+  if constexpr (NQ == 4) {
+    box_muller2(a[0], a[1], a[2], a[3], z0);
+    box_muller2(b[0], b[1], b[2], b[3], z1);
   } else {
-    const float4 z = vbt_normal_quad(P.seed, tj, 0u, kVbtRoot, quad);
-    if (L <= kVbtCacheLevels) {
-      C.traj = (long long)traj;
+    float z[4];
+    box_muller2(sel ? a[2] : a[0], sel ? a[3] : a[1], sel ? b[2] : b[0], sel ? b[3] : b[1], z);
+    z0[0] = z[0];
+    z0[1] = z[1];
+    z1[0] = z[2];
+    z1[1] = z[3];
+  }
+}
+
+// The bridge state of one descent path for NQ dimensions: W at the start of each
+// level's dyadic interval and the increment across it.  Consecutive evaluations of
+// a solve lie close together, so their paths share the upper levels; an evaluation
+// re-descends only below the deepest level whose interval also contains the new
+// time.
+constexpr int kVbtCacheLevels = 24;
+template <int NQ>
+struct VbtCache {
+  float ws[kVbtCacheLevels + 1][NQ], wsu[kVbtCacheLevels + 1][NQ];
+  uint32_t node;   // heap index of the cached path's leaf interval
+  long long traj;  // trajectory of the cached path (-1: none)
+};
+using VbtQuadCache = VbtCache<4>;
+
+// sqrt(T) W_unit(r) for NQ dimensions of trajectory `traj` at time t, by the descent
+// of tree.py:406-409, 607-621, 752-768: at every level the path takes the half that
+// holds r (the left one at its midpoint), down to 2^-level <= tol.  The path is known
+// from r alone, so the levels' normals are drawn two at a time (the leaf's with the
+// last) and the short bridge recursion follows.  C (may be null): the cached path.
+// Bound: issue slots, ~96 a warp and Philox block and ~112 a pair of Box--Muller
+// pairs.  The Ornstein--Uhlenbeck solve of 16384 paths and 100 steps (under one warp
+// a scheduler, so the overlapped draws count most) went from 0.82 to 0.49 ms, the
+// neural SDE of 32768 from 3.75 to 3.64 ms, its gradient at 9001 from 9.0 to 8.5 ms.
+template <int NQ>
+__device__ __forceinline__ void vbt_w(const SolveParams &P, int64_t traj, double t, int quad,
+                                      int sel, VbtCache<NQ> *C, float (&w)[NQ]) {
+  const float r = float((t - P.vbt_t0) * P.vbt_inv_len);
+  const uint32_t tj = uint32_t(traj);
+  const int L = P.vbt_levels;
+  uint32_t node;
+  float su, f;  // the leaf interval's length, and r's place in it over its length
+  if (L <= 30) {
+    // r lies in (i 2^-L, (i + 1) 2^-L]; scaling by 2^L is exact, and from 2^24 on
+    // the scaled r is an integer, the interval's end
+    const float x = r * __int_as_float((127 + L) << 23);
+    su = __int_as_float((127 - L) << 23);
+    const int i = max(0, min(int(ceilf(x)) - 1, (1 << L) - 1));
+    node = (1u << L) + uint32_t(i);
+    f = fmaxf(x < 16777216.f ? x - float(i) : 1.f, 0.f);
+  } else {
+    float s = 0.f;
+    su = 1.f;
+    node = 1;
+    for (int l = 0; l < L; l++) {
+      su *= 0.5f;
+      const bool right = r > s + su;
+      if (right) s += su;
+      node = 2 * node + (right ? 1u : 0u);
+    }
+    f = fmaxf(r - s, 0.f) / su;
+  }
+  float ws[NQ], wsu[NQ];
+  int d = 0;
+  const bool cached = C && L <= kVbtCacheLevels;
+  if (cached && C->traj == (long long)traj) {
+    const uint32_t x = node ^ C->node;
+    d = x == 0 ? L : L - 1 - (31 - __clz(x));  // levels shared with the cached path
 #pragma unroll
-      for (int q = 0; q < 4; q++) C.ws[0][q] = 0.f;
-      C.wsu[0][0] = z.x;
-      C.wsu[0][1] = z.y;
-      C.wsu[0][2] = z.z;
-      C.wsu[0][3] = z.w;
+    for (int q = 0; q < NQ; q++) {
+      ws[q] = C->ws[d][q];
+      wsu[q] = C->wsu[d][q];
+    }
+  } else {
+    float unused[NQ];
+    vbt_normals2<NQ>(P.seed, tj, 0u, kVbtRoot, 0u, kVbtRoot, quad, sel, wsu, unused);
+#pragma unroll
+    for (int q = 0; q < NQ; q++) ws[q] = 0.f;
+    if (cached) {
+      C->traj = (long long)traj;
+#pragma unroll
+      for (int q = 0; q < NQ; q++) {
+        C->ws[0][q] = 0.f;
+        C->wsu[0][q] = wsu[q];
+      }
     }
   }
-  float ws[4], wsu[4];
-  if (L <= kVbtCacheLevels) {
+  // one level: the halves of the interval of level l, and the one with r
+  auto descend = [&](int l, const float (&z)[NQ]) {
+    // sqrt(2^-l) / 2
+    const float a = __int_as_float((126 - ((l + 1) >> 1)) << 23) * (l & 1 ? 1.41421354f : 1.f);
+    const bool right = (node >> (L - l - 1)) & 1u;
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
-      ws[q] = C.ws[d][q];
-      wsu[q] = C.wsu[d][q];
-    }
-  } else {  // deeper than the cache: plain descent from the root
-    const float4 z = vbt_normal_quad(P.seed, tj, 0u, kVbtRoot, quad);
-    ws[0] = ws[1] = ws[2] = ws[3] = 0.f;
-    wsu[0] = z.x;
-    wsu[1] = z.y;
-    wsu[2] = z.z;
-    wsu[3] = z.w;
-  }
-  // replay the first d decisions for the interval at level d
-  s = 0.f;
-  su = 1.f;
-  for (int l = 0; l < d; l++) {
-    const float st = 0.5f * su, tm = s + st;
-    if (r > tm) s = tm;
-    su = st;
-  }
-  for (int l = d; l < L; l++) {
-    const float st = 0.5f * su, tm = s + st;
-    const float4 z = vbt_normal_quad(P.seed, tj, node >> (L - l), kVbtMid, quad);
-    const float a = 0.5f * sqrtf(su);
-    const float zz[4] = {z.x, z.y, z.z, z.w};
-    const bool right = r > tm;
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
+    for (int q = 0; q < NQ; q++) {
       const float m = 0.5f * wsu[q];
-      const float wst = m + a * zz[q], wtu = m - a * zz[q];
-      if (right) {
-        ws[q] += wst;
-        wsu[q] = wtu;
-      } else {
-        wsu[q] = wst;
-      }
+      const float wst = m + a * z[q], wtu = m - a * z[q];
+      if (right) ws[q] += wst;
+      wsu[q] = right ? wtu : wst;
     }
-    if (right) s = tm;
-    su = st;
-    if (l + 1 <= kVbtCacheLevels) {
+    if (cached) {
 #pragma unroll
-      for (int q = 0; q < 4; q++) {
-        C.ws[l + 1][q] = ws[q];
-        C.wsu[l + 1][q] = wsu[q];
+      for (int q = 0; q < NQ; q++) {
+        C->ws[l + 1][q] = ws[q];
+        C->wsu[l + 1][q] = wsu[q];
       }
     }
+  };
+  float z0[NQ], z1[NQ];
+  int l = d;
+#pragma unroll 1
+  for (; l < L; l += 2) {
+    const bool leaf = l + 1 == L;
+    vbt_normals2<NQ>(P.seed, tj, node >> (L - l), kVbtMid, node >> (L - l - 1),
+                     leaf ? kVbtLeaf : kVbtMid, quad, sel, z0, z1);
+    descend(l, z0);
+    if (!leaf) descend(l + 1, z1);
   }
-  C.node = node;
-  const float sr = fmaxf(r - s, 0.f), ru = fmaxf(su - sr, 0.f);
-  const float4 z = vbt_normal_quad(P.seed, tj, node, kVbtLeaf, quad);
-  const float bb = sqrtf(sr * ru / su), f = sr / su;
+  if (l == L) vbt_normals2<NQ>(P.seed, tj, node, kVbtLeaf, node, kVbtLeaf, quad, sel, z1, z0);
+  if (cached) C->node = node;
+  float bb;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(bb) : "f"(f * fmaxf(1.f - f, 0.f) * su));
   const float sq = P.vbt_sqrt_len;
-  return make_float4(sq * (ws[0] + f * wsu[0] + bb * z.x), sq * (ws[1] + f * wsu[1] + bb * z.y),
-                     sq * (ws[2] + f * wsu[2] + bb * z.z), sq * (ws[3] + f * wsu[3] + bb * z.w));
+#pragma unroll
+  for (int q = 0; q < NQ; q++) w[q] = sq * (ws[q] + f * wsu[q] + bb * z1[q]);
+}
+
+// Dimensions (col, col + 1).
+static __device__ __noinline__ float2 vbt_w_pair(const SolveParams &P, int64_t traj, double t,
+                                                 int col) {
+  float w[2];
+  vbt_w<2>(P, traj, t, col >> 2, col & 2, nullptr, w);
+  return make_float2(w[0], w[1]);
+}
+
+// A quad of dimensions 4 quad .. 4 quad + 3, from the cached path.
+static __device__ __noinline__ float4 vbt_w_quad(const SolveParams &P, int64_t traj, double t,
+                                                 int quad, VbtQuadCache &C) {
+  float w[4];
+  vbt_w<4>(P, traj, t, quad, 0, &C, w);
+  return make_float4(w[0], w[1], w[2], w[3]);
 }
 
 // The tree with space-time Levy area: W_unit(r) and bar H_unit(r) = r H_{0,r}
