@@ -242,6 +242,13 @@ struct BsField {
     *reinterpret_cast<float2 *>(rec + row * REC + roff + col) = make_float2(v0, v1);
   }
 
+  __device__ static __forceinline__ void put_hidden(Sm &sm, int which, int row, int col, F2 v,
+                                                    float *rec, int roff) {
+    float v0, v1;
+    f2_unpack(v, v0, v1);
+    put_hidden(sm, which, row, col, v0, v1, rec, roff);
+  }
+
   // F = MLP(X) and GY = A^T dMLP/dX (owned layout) with the stage records.
   // X and G must have been written and synchronised.  Ends with every warp
   // past its last read of R1 only after the caller's next barrier.
@@ -325,9 +332,9 @@ struct BsField {
         for (int j = 0; j < SH::TPWH; j++) {
           const int col = (nth0 + j) * 8 + 2 * c, r0 = mth * 16 + g;
           const float bb0 = sm.b0[col], bb1 = sm.b0[col + 1];
-          put_hidden(sm, 1, r0, col, tanhf(acc[j][0] + bb0), tanhf(acc[j][1] + bb1), rec,
+          put_hidden(sm, 1, r0, col, tanh2(acc[j][0] + bb0, acc[j][1] + bb1), rec,
                      SH::RH1);
-          put_hidden(sm, 1, r0 + 8, col, tanhf(acc[j][2] + bb0), tanhf(acc[j][3] + bb1), rec,
+          put_hidden(sm, 1, r0 + 8, col, tanh2(acc[j][2] + bb0, acc[j][3] + bb1), rec,
                      SH::RH1);
         }
       }
@@ -343,9 +350,9 @@ struct BsField {
         for (int j = 0; j < SH::TPWH; j++) {
           const int col = (nth0 + j) * 8 + 2 * c, r0 = mth * 16 + g;
           const float bb0 = sm.b1[col], bb1 = sm.b1[col + 1];
-          put_hidden(sm, 2, r0, col, tanhf(acc[j][0] + bb0), tanhf(acc[j][1] + bb1), rec,
+          put_hidden(sm, 2, r0, col, tanh2(acc[j][0] + bb0, acc[j][1] + bb1), rec,
                      SH::RH2);
-          put_hidden(sm, 2, r0 + 8, col, tanhf(acc[j][2] + bb0), tanhf(acc[j][3] + bb1), rec,
+          put_hidden(sm, 2, r0 + 8, col, tanh2(acc[j][2] + bb0, acc[j][3] + bb1), rec,
                      SH::RH2);
         }
       }

@@ -257,9 +257,9 @@ struct MlpField {
           const int col = (nt0 + j) * 8 + 2 * c, r0 = mt * 16 + g;
           const float bb0 = sm.b0[col], bb1 = sm.b0[col + 1];
           __nv_bfloat16 *p2a = sm.a1l2(r0), *p2b = sm.a1l2(r0 + 8);
-          store_split3x2(tanhf(acc[j][0] + bb0), tanhf(acc[j][1] + bb1), &sm.A1[r0][col],
+          store_split3x2(tanh2(acc[j][0] + bb0, acc[j][1] + bb1), &sm.A1[r0][col],
                          &sm.A1l[r0][col], p2a ? p2a + col : nullptr);
-          store_split3x2(tanhf(acc[j][2] + bb0), tanhf(acc[j][3] + bb1), &sm.A1[r0 + 8][col],
+          store_split3x2(tanh2(acc[j][2] + bb0, acc[j][3] + bb1), &sm.A1[r0 + 8][col],
                          &sm.A1l[r0 + 8][col], p2b ? p2b + col : nullptr);
         }
       }
@@ -271,10 +271,13 @@ struct MlpField {
         split_gemm<D, SH::TPW>(acc, &sm.X[mt * 16][0], &sm.Xl[mt * 16][0], sm.xl2(mt * 16),
                                SH::PD, &sm.Ws[nt0 * 8][0], SH::PD, lane);
 #pragma unroll
-        for (int e = 0; e < NE; e++) {
+        for (int e = 0; e < NE; e += 2) {
           int row, col;
           elem_rc<SH>(e, warp, lane, row, col);
-          sig[e] = 0.1f * tanhf(acc[e >> 2][e & 3] + sm.bs[col]);
+          f2_unpack(f2_mul(tanh2(acc[e >> 2][e & 3] + sm.bs[col],
+                                 acc[e >> 2][(e & 3) + 1] + sm.bs[col + 1]),
+                           f2_set(0.1f)),
+                    sig[e], sig[e + 1]);
         }
       }
       __syncthreads();
@@ -292,9 +295,9 @@ struct MlpField {
           const int col = (nt0 + j) * 8 + 2 * c, r0 = mt * 16 + g;
           const float bb0 = sm.b1[col], bb1 = sm.b1[col + 1];
           __nv_bfloat16 *p2a = sm.a2l2r(r0), *p2b = sm.a2l2r(r0 + 8);
-          store_split3x2(tanhf(acc[j][0] + bb0), tanhf(acc[j][1] + bb1), &A2[r0][col],
+          store_split3x2(tanh2(acc[j][0] + bb0, acc[j][1] + bb1), &A2[r0][col],
                          &A2l[r0][col], p2a ? p2a + col : nullptr);
-          store_split3x2(tanhf(acc[j][2] + bb0), tanhf(acc[j][3] + bb1), &A2[r0 + 8][col],
+          store_split3x2(tanh2(acc[j][2] + bb0, acc[j][3] + bb1), &A2[r0 + 8][col],
                          &A2l[r0 + 8][col], p2b ? p2b + col : nullptr);
         }
       }

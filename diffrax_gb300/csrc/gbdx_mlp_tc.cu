@@ -261,7 +261,8 @@ __device__ __forceinline__ void hidden_epilogue(TcSmem &sm, uint32_t lane_addr, 
     float v[16];
     tc::tmem_ld16(lane_addr + kAcc + c, v);
 #pragma unroll
-    for (int j = 0; j < 16; j++) v[j] = tanhf(v[j] + b[c + j]);
+    for (int j = 0; j < 16; j += 2)
+      f2_unpack(tanh2(v[j] + b[c + j], v[j + 1] + b[c + j + 1]), v[j], v[j + 1]);
     put16(sm, row, c, kH, v);
   }
 }

@@ -10,6 +10,8 @@
 #include <cuda_bf16.h>
 #include <stdint.h>
 
+#include "gbdx_f2.cuh"
+
 namespace gbdx {
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
@@ -131,6 +133,13 @@ __device__ __forceinline__ void store_split3x2(float x0, float x1, __nv_bfloat16
     const float2 mf = __bfloat1622float2(m);
     *reinterpret_cast<__nv_bfloat162 *>(p2) = __floats2bfloat162_rn(r0 - mf.x, r1 - mf.y);
   }
+}
+
+__device__ __forceinline__ void store_split3x2(F2 x, __nv_bfloat16 *p0, __nv_bfloat16 *p1,
+                                               __nv_bfloat16 *p2) {
+  float x0, x1;
+  f2_unpack(x, x0, x1);
+  store_split3x2(x0, x1, p0, p1, p2);
 }
 
 // Two adjacent values as hi/lo BF16x2 words.
