@@ -669,7 +669,8 @@ def diffeqsolve(terms, solver, t0, t1, dt0, y0, args=None, *,
 
     Extra keyword arguments select the GB300 execution policy: ``kernel`` is
     "fused" (persistent work-stealing integrator, the default), "plain" (one
-    trajectory per thread) or "tc" (MLP-field forward on tcgen05 tensor cores); ``block_threads`` / ``ctas_per_sm`` override the
+    trajectory per thread) or "tc" (the MLP-field forward on the tcgen05 tensor
+    cores by name; "fused" runs it too); ``block_threads`` / ``ctas_per_sm`` override the
     autotuned launch shape of the fused kernel; ``schedule`` ("auto",
     "index", "longest_first") sets the order in which the fused kernel takes
     trajectories (results do not depend on it); ``autotune=True`` times a few

@@ -48,9 +48,9 @@ def _key(fields: dict, batch: int):
 
 
 def tc_eligible(fields: dict) -> bool:
-    """Whether the tcgen05 forward (kernel "tc") serves this problem: BF16
-    forward solves of 64 -> 128 -> 128 -> 64 MLP ODE fields with Tsit5 or
-    Dopri5."""
+    """Whether kernel "tc" (the tcgen05 forward asked for by name; "fused" runs
+    the same one) serves this problem: BF16 forward solves of 64 -> 128 -> 128
+    -> 64 MLP ODE fields with Tsit5 or Dopri5."""
     return (fields.get("field") == 3 and fields.get("solver") in (2, 3) and
             tuple(fields.get("mlp_widths", ())) == (64, 128, 128, 64) and
             fields.get("mlp_precision", 0) == 0 and fields.get("adjoint", 0) == 0 and
@@ -61,8 +61,8 @@ def tc_eligible(fields: dict) -> bool:
 
 def candidates(fields: dict, batch: int) -> list:
     """(kernel, block_threads, ctas_per_sm) shapes worth timing for this
-    problem: the launch shape of the fused kernels and, for the MLP fields,
-    the tile shape (32-row mma.sync tiles, or 128-row tcgen05 tiles)."""
+    problem: the launch shape of the fused kernels (of the MLP fields, the CTAs
+    per SM)."""
     kernel = fields.get("kernel", 0)
     if fields.get("field") == 3:  # MLP fields: one row tile per CTA
         out = [("fused", 0, c) for c in (1, 2, 3, 4)]

@@ -66,8 +66,8 @@ struct gbdx_problem {
   gbdx::BsEntry bs;    // BacksolveAdjoint backward (MLP fields)
   gbdx::AdjEntry adj;  // gradients of the analytic fields (y0 and args)
   bool mlp;            // MLP-field row-tile integrator
+  int fm_rows;         // rows per tile of its feature-major tcgen05 form (0: not that form)
   int rows_per_cta;
-  int mlp_block;       // threads per CTA of the MLP integrator
 };
 
 namespace gbdx {
@@ -81,8 +81,7 @@ namespace {
 // Workspace of one solve: the work counter, the work order, and (recursive
 // adjoint) the tape the backward reads plus its scratch.
 struct WsLayout {
-  size_t order, ffrag, tape_t, tape_y, tape_n, tape_s, scratch, psum, pcomp, bounds, total;
-  bool has_ffrag;  // width-256 MLP forward: W0 / W2 fragments at ffrag
+  size_t order, tape_t, tape_y, tape_n, tape_s, scratch, psum, pcomp, bounds, total;
   size_t frag, rec, ath;  // backsolve: B fragments, stage records, a_theta
   int seg_max, n_cta;
   bool track;
@@ -102,11 +101,6 @@ int ws_layout(const gbdx_problem *p, int64_t batch, WsLayout *L) {
   L->order = off;
   if (d.kernel != GBDX_KERNEL_PLAIN && d.schedule != GBDX_SCHED_INDEX)
     off += up256(gbdx::schedule_workspace_bytes(int64_t(B)));
-  // The width-256 MLP integrator reads W0 and W2 as BF16 mma fragments.
-  L->ffrag = off;
-  L->has_ffrag = p->mlp && d.kernel != GBDX_KERNEL_TC && d.mlp_widths[1] >= 256 &&
-                 d.mlp_precision != GBDX_MLP_FP32;
-  if (L->has_ffrag) off += 2 * up256(size_t(d.dim) * d.mlp_widths[1] * 2);
   L->tape_t = L->tape_y = L->tape_n = L->tape_s = L->scratch = L->psum = L->pcomp = off;
   L->seg_max = 0;
   L->n_cta = 0;
@@ -412,8 +406,8 @@ int gbdx_problem_create(const gbdx_problem_desc *desc, gbdx_problem **out) {
   p->bs = gbdx::BsEntry{nullptr, nullptr, 0, 0, 0, 0};
   p->adj = gbdx::AdjEntry{};
   p->mlp = false;
+  p->fm_rows = 0;
   p->rows_per_cta = 1;
-  p->mlp_block = 256;
   if (d.n_step_ts < 0 || d.n_jump_ts < 0) {
     delete p;
     return fail(GBDX_ERR_INVALID, "negative number of step_ts or jump_ts");
@@ -555,7 +549,8 @@ int gbdx_problem_create(const gbdx_problem_desc *desc, gbdx_problem **out) {
         return fail(GBDX_ERR_UNSUPPORTED,
                     "the tensor-core (TC) kernel runs BF16 forward solves without an adjoint");
       }
-      p->ode = gbdx::find_mlp_tc_entry(d.solver, D, H, sde);
+      if (D == 64 && H == 128 && !sde && (d.solver == GBDX_TSIT5 || d.solver == GBDX_DOPRI5))
+        p->ode = gbdx::find_mlp_fm_entry_d64h128(d.solver);
       if (!p->ode.launch) {
         delete p;
         return fail(GBDX_ERR_UNSUPPORTED,
@@ -564,8 +559,7 @@ int gbdx_problem_create(const gbdx_problem_desc *desc, gbdx_problem **out) {
                     sde ? ", SDE" : "");
       }
       p->mlp = true;
-      p->rows_per_cta = 128;
-      p->mlp_block = 512;  // four threads per trajectory
+      p->fm_rows = 32;
       *out = p;
       return GBDX_OK;
     }
@@ -608,6 +602,23 @@ int gbdx_problem_create(const gbdx_problem_desc *desc, gbdx_problem **out) {
     if (D == 32 && H == 64) {
       p->ode_xo = gbdx::find_mlp_xo_entry_d32h64(d.solver, precise, sde);
       p->ode = xo ? p->ode_xo : gbdx::find_mlp_entry_d32h64(d.solver, precise, sde);
+    }
+    if (!precise && !sde) {
+      // BF16 ODEs: the feature-major tcgen05 form
+      if (D == 64 && H == 128) {
+        p->ode_xo = gbdx::find_mlp_fm_xo_entry_d64h128(d.solver);
+        p->ode = gbdx::find_mlp_fm_entry_d64h128(d.solver);
+      }
+      if (D == 64 && H == 256) {
+        p->ode_xo = gbdx::find_mlp_fm_xo_entry_d64h256(d.solver);
+        p->ode = gbdx::find_mlp_fm_entry_d64h256(d.solver);
+      }
+      if (D == 32 && H == 64) {
+        p->ode_xo = gbdx::find_mlp_fm_xo_entry_d32h64(d.solver);
+        p->ode = gbdx::find_mlp_fm_entry_d32h64(d.solver);
+      }
+      if (xo) p->ode = p->ode_xo;
+      p->fm_rows = 32;
     }
     if (!p->ode.launch) {
       delete p;
@@ -893,24 +904,9 @@ static int solve_fwd(const gbdx_problem *problem, int64_t batch, const double *t
     P.saves_prefilled = 1;
   }
 
-  if (L.has_ffrag) {
-    // W0 (B[k][n] = W0[n][k], K = D, N = H) and W2 (K = H, N = D) as BF16
-    // mma fragments for this launch
-    const int D = d.dim, H = d.mlp_widths[1];
-    const float *W = static_cast<const float *>(params);
-    uint2 *f0 = reinterpret_cast<uint2 *>(static_cast<char *>(workspace) + L.ffrag);
-    uint2 *f2 = reinterpret_cast<uint2 *>(static_cast<char *>(workspace) + L.ffrag +
-                                          up256(size_t(D) * H * 2));
-    cudaError_t e = gbdx::launch_frag_prep(W, D, D, H, 1, f0, s);
-    if (e == cudaSuccess)
-      e = gbdx::launch_frag_prep(W + size_t(H) * D + H + size_t(H) * H + H, H, H, D, 1, f2, s);
-    if (e != cudaSuccess) return cuda_fail(e, "weight fragments");
-    P.w0f = f0;
-    P.w2f = f2;
-  }
   gbdx::LaunchCfg cfg;
   cfg.kernel = d.kernel == GBDX_KERNEL_PLAIN ? GBDX_KERNEL_PLAIN : GBDX_KERNEL_FUSED;
-  cfg.block = problem->mlp ? problem->mlp_block : (d.block_threads > 0 ? d.block_threads : 64);
+  cfg.block = d.block_threads > 0 ? d.block_threads : 64;
   if (!problem->mlp && (cfg.block % 32 != 0 || cfg.block > 256))
     return fail(GBDX_ERR_INVALID, "block_threads must be a multiple of 32 up to 256");
   cfg.grid = 1;
@@ -923,7 +919,7 @@ static int solve_fwd(const gbdx_problem *problem, int64_t batch, const double *t
     if (e != cudaSuccess) return cuda_fail(e, "occupancy query");
     if (occ < 1) occ = 1;
     int per_sm = d.ctas_per_sm;
-    if (per_sm <= 0 && problem->mlp) per_sm = occ;
+    if (problem->mlp && (per_sm <= 0 || (problem->fm_rows && per_sm > occ))) per_sm = occ;
     if (per_sm <= 0) {
       // Keep about B / 1.7 lanes resident: enough warps to hide the step's
       // dependency latency, few enough that lanes refill from the queue and
@@ -934,7 +930,9 @@ static int solve_fwd(const gbdx_problem *problem, int64_t batch, const double *t
       if (per_sm > occ) per_sm = occ;
     }
     int64_t grid = (int64_t)sms * per_sm;
-    const int rows = problem->mlp ? problem->rows_per_cta : cfg.block;
+    const int rows = problem->fm_rows ? problem->fm_rows
+                     : problem->mlp   ? problem->rows_per_cta
+                                      : cfg.block;
     const int64_t needed = (batch + rows - 1) / rows;
     if (grid > needed) grid = needed;
     cfg.grid = (int)grid;

@@ -37,10 +37,6 @@ struct MlpShape {
   static constexpr int D = D_, H = H_;
   static constexpr int M = (H_ >= 256) ? 16 : 32;  // rows per CTA
   static constexpr int THREADS = 256, WARPS = 8;
-  // Width 256: W0 and W2 are read as pre-arranged BF16 mma B fragments from
-  // global memory (L2-resident, 32 KB each), so that W1 and the three-piece
-  // activations fit the 227 KB of shared memory.
-  static constexpr bool GFRAG = H_ >= 256;
   static constexpr int PD = D + 8, PH = H + 8;      // padded smem row strides (bf16)
   static constexpr int PW0 = D + 8;                 // row stride of W0
   static constexpr int MT = M / 16, NT = D / 8, NTH = H / 8;
@@ -69,24 +65,24 @@ struct RowState {
   double ginv[M];  // RN(1 / nc), for the grid fraction
   int sdown[M], stslot[M];  // SaveAt(steps=n): steps to the next save; this step's slot
   int sidx[M], jidx[M];     // ClipStepSizeController: search hints into step_ts / jump_ts
-  // the error norm's partial sums per 8-column output tile, added in a fixed
-  // order (results do not depend on warp timing)
-  float part[M][8];
 };
 
-// Events (registered conditions) of the extended-output integrator, in the
-// dynamic shared memory after the kernel's own: the conditions' last values,
-// the one that fired (-1: none), the event time, the latest time a save may
-// take (the event time once a root was found), the root's theta in its step
-// (-1: no root); components 0..3 of y0, y1 and the stage increments for the
-// root find; the steady-state norms' per-tile partials (f.f, y.y).
+// Events (registered conditions) of the extended-output integrators: the
+// conditions' last values, the one that fired (-1: none), the event time, the
+// latest time a save may take (the event time once a root was found), the root's
+// theta in its step (-1: no root).
 template <int M>
 struct RowEvents {
   double evv[M][GBDX_MAX_EVENTS], tfin[M], tsave[M];
   int evi[M];
   float thfin[M];
+};
+// A step's scratch for them: components 0..3 of y0, y1 and the stage increments
+// for the root find; NPART partial sums of the steady-state norms (f.f, y.y).
+template <int M, int NPART>
+struct RowEventStep {
   float ey0[M][4], ey1[M][4], ek[M][7][4];
-  float pf[M][8], py[M][8];
+  float pf[M][NPART], py[M][NPART];
 };
 
 template <class SH, bool PRECISE, bool SDE>
@@ -95,10 +91,9 @@ struct MlpSmem;
 template <class SH, bool SDE>
 struct MlpSmem<SH, false, SDE> {
   static constexpr int M3 = SH::NP == 3 ? SH::M : 1;
-  __nv_bfloat16 W0[SH::GFRAG ? 1 : SH::H][SH::PW0];  // (global fragments at width 256)
+  __nv_bfloat16 W0[SH::H][SH::PW0];
   __nv_bfloat16 W1[SH::H][SH::PH];
-  __nv_bfloat16 W2[SH::GFRAG ? 1 : SH::D][SH::PH];
-  const uint2 *w0f, *w2f;                            // the fragments (width 256)
+  __nv_bfloat16 W2[SH::D][SH::PH];
   __nv_bfloat16 Ws[SDE ? SH::D : 1][SH::PD];
   float b0[SH::H], b1[SH::H], b2[SH::D], bs[SH::D];
   // stage input and hidden activations as BF16 pieces (the third piece only
@@ -107,6 +102,9 @@ struct MlpSmem<SH, false, SDE> {
   __nv_bfloat16 A1[SH::M][SH::PH], A1l[SH::M][SH::PH], A1l2[M3][SH::PH];
   __nv_bfloat16 A2s[SH::M][SH::PH], A2ls[SH::M][SH::PH], A2l2s[M3][SH::PH];
   RowState<SH::M> rows;
+  // the error norm's partial sums per 8-column output tile, added in a fixed
+  // order (results do not depend on warp timing)
+  float part[SH::M][8];
   __device__ __nv_bfloat16 (*a2())[SH::PH] { return A2s; }
   __device__ __nv_bfloat16 (*a2l())[SH::PH] { return A2ls; }
   __device__ __nv_bfloat16 (*a2l2())[SH::PH] { return A2l2s; }
@@ -123,6 +121,7 @@ struct MlpSmem<SH, true, SDE> {
   float A1[SH::M][SH::H + 1];
   float A2[SH::M][SH::H + 1];
   RowState<SH::M> rows;
+  float part[SH::M][8];
 };
 
 // (row, col) of owned element e of this thread in the output-tile layout.
@@ -140,8 +139,7 @@ struct MlpField {
   using Sm = MlpSmem<SH, PRECISE, SDE>;
   static constexpr int D = SH::D, H = SH::H, M = SH::M, NE = SH::NE;
 
-  // Stage the weights (BF16 mode) and biases into shared memory (at width 256
-  // only W1: W0 and W2 are the global fragments S.w0f, S.w2f).
+  // Stage the weights (BF16 mode) and biases into shared memory.
   __device__ static void stage(Sm &sm, const SolveParams &S, int tid) {
     const float *P = S.mlp;
     for (int i = tid; i < H; i += SH::THREADS) {
@@ -154,17 +152,10 @@ struct MlpField {
     }
     if constexpr (!PRECISE) {
       // the model's BF16 weights
-      if constexpr (SH::GFRAG) {
-        if (tid == 0) {
-          sm.w0f = S.w0f;
-          sm.w2f = S.w2f;
-        }
-      } else {
-        for (int i = tid; i < H * D; i += SH::THREADS)
-          sm.W0[i / D][i % D] = __float2bfloat16_rn(P[SH::OW0 + i]);
-        for (int i = tid; i < D * H; i += SH::THREADS)
-          sm.W2[i / H][i % H] = __float2bfloat16_rn(P[SH::OW2 + i]);
-      }
+      for (int i = tid; i < H * D; i += SH::THREADS)
+        sm.W0[i / D][i % D] = __float2bfloat16_rn(P[SH::OW0 + i]);
+      for (int i = tid; i < D * H; i += SH::THREADS)
+        sm.W2[i / H][i % H] = __float2bfloat16_rn(P[SH::OW2 + i]);
       for (int i = tid; i < H * H; i += SH::THREADS)
         sm.W1[i / H][i % H] = __float2bfloat16_rn(P[SH::OW1 + i]);
       if constexpr (SDE)
@@ -246,12 +237,8 @@ struct MlpField {
         float acc[SH::TPWH][4];
 #pragma unroll
         for (int j = 0; j < SH::TPWH; j++) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
-        if constexpr (SH::GFRAG)
-          gemm_gfrag_p<D, SH::TPWH, SH::NP>(acc, &sm.X[mt * 16][0], &sm.Xl[mt * 16][0],
-                                            sm.xl2(mt * 16), SH::PD, sm.w0f, nt0, lane);
-        else
-          split_gemm<D, SH::TPWH>(acc, &sm.X[mt * 16][0], &sm.Xl[mt * 16][0], sm.xl2(mt * 16),
-                                  SH::PD, &sm.W0[nt0 * 8][0], SH::PW0, lane);
+        split_gemm<D, SH::TPWH>(acc, &sm.X[mt * 16][0], &sm.Xl[mt * 16][0], sm.xl2(mt * 16),
+                                SH::PD, &sm.W0[nt0 * 8][0], SH::PW0, lane);
 #pragma unroll
         for (int j = 0; j < SH::TPWH; j++) {
           const int col = (nt0 + j) * 8 + 2 * c, r0 = mt * 16 + g;
@@ -307,12 +294,8 @@ struct MlpField {
         float acc[SH::TPW][4];
 #pragma unroll
         for (int j = 0; j < SH::TPW; j++) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
-        if constexpr (SH::GFRAG)
-          gemm_gfrag_p<H, SH::TPW, SH::NP>(acc, &sm.a2()[mt * 16][0], &sm.a2l()[mt * 16][0],
-                                           sm.a2l2r(mt * 16), SH::PH, sm.w2f, nt0, lane);
-        else
-          split_gemm<H, SH::TPW>(acc, &sm.a2()[mt * 16][0], &sm.a2l()[mt * 16][0],
-                                 sm.a2l2r(mt * 16), SH::PH, &sm.W2[nt0 * 8][0], SH::PH, lane);
+        split_gemm<H, SH::TPW>(acc, &sm.a2()[mt * 16][0], &sm.a2l()[mt * 16][0],
+                               sm.a2l2r(mt * 16), SH::PH, &sm.W2[nt0 * 8][0], SH::PH, lane);
 #pragma unroll
         for (int e = 0; e < NE; e++) {
           int row, col;
@@ -644,7 +627,7 @@ __device__ __forceinline__ bool mlp_ev_fires(const SolveParams &P, int e, double
 // Per-tile partial sums of f.f and y.y of every row (the steady-state
 // condition's norms, _event.py:120-175), one slot per 8-column tile.
 template <class SH, int M, int NE>
-__device__ __forceinline__ void steady_partials(RowEvents<M> &R, const float (&F)[NE],
+__device__ __forceinline__ void steady_partials(RowEventStep<M, 8> &R, const float (&F)[NE],
                                                 const float (&Y)[NE], int warp, int lane) {
 #pragma unroll
   for (int j = 0; j < SH::TPW; j++) {
@@ -671,17 +654,18 @@ __device__ __forceinline__ void steady_partials(RowEvents<M> &R, const float (&F
   }
 }
 
-// Value of steady-state condition e for row r from its partials.
-template <class SH, int M>
-__device__ __forceinline__ double steady_value(const SolveParams &P, const RowEvents<M> &R, int r,
-                                               int e) {
+// Value of steady-state condition e for row r of a D-dimensional state from its
+// partials, N of them in use.
+template <int D, int N, int M, int NPART>
+__device__ __forceinline__ double steady_value(const SolveParams &P,
+                                               const RowEventStep<M, NPART> &R, int r, int e) {
   float sf = 0.f, sy = 0.f;
 #pragma unroll
-  for (int n = 0; n < SH::NT; n++) {
+  for (int n = 0; n < N; n++) {
     sf += R.pf[r][n];
     sy += R.py[r][n];
   }
-  return sqrt(double(sf) / SH::D) < P.ev_coef[6 * e + 1] + P.ev_coef[6 * e] * sqrt(double(sy) / SH::D)
+  return sqrt(double(sf) / D) < P.ev_coef[6 * e + 1] + P.ev_coef[6 * e] * sqrt(double(sy) / D)
              ? 1.0
              : 0.0;
 }
@@ -740,8 +724,8 @@ __device__ __forceinline__ float mlp_interp(float th, float y0, float y1, const 
 // g(t) = w . interp(t) + wt t + c over [tp, tn] from t = tn, each iterate
 // clipped to the step; components 0..3 of the step's y0, y1 and stages come
 // from the row state.  Returns the root; ok = false after 256 iterations.
-template <int SOLVER, int S, int M>
-__device__ double mlp_ev_root(const SolveParams &P, const RowEvents<M> &R, int r,
+template <int SOLVER, int S, int M, int NPART>
+__device__ double mlp_ev_root(const SolveParams &P, const RowEventStep<M, NPART> &R, int r,
                               const double (&cf)[6], int nc, double tp, double tn, bool &ok) {
   ok = true;
   const double span = tn - tp;
@@ -774,6 +758,54 @@ __device__ double mlp_ev_root(const SolveParams &P, const RowEvents<M> &R, int r
   return t;
 }
 
+// The conditions of row r at the state an accepted step ended in: the first (in
+// order) that fires ends the solve, at the root inside the step with a root finder.
+template <int SOLVER, int S, int D, int N, int M, int NPART>
+__device__ void row_events(RowState<M> &R, RowEvents<M> &E, const RowEventStep<M, NPART> &ES,
+                           int r, const SolveParams &P) {
+  const double tn = R.tn_old[r], tp = R.tp_old[r];
+  int fired = -1;
+#pragma unroll
+  for (int e = 0; e < GBDX_MAX_EVENTS; e++) {
+    if (e < P.n_event) {
+      double v;
+      if (P.ev_kind[e] == GBDX_EV_STEADY) {
+        v = steady_value<D, N>(P, ES, r, e);
+      } else {
+        v = 0.0;
+        for (int n = 0; n < (D < 4 ? D : 4); n++)
+          v += P.ev_coef[6 * e + n] * double(ES.ey1[r][n]);
+        v += P.ev_coef[6 * e + 4] * tn;
+        v += P.ev_coef[6 * e + 5];
+        if (P.ev_kind[e] == GBDX_EV_LINEAR_BOOL) v = v > 0 ? 1.0 : 0.0;
+      }
+      if (fired < 0 && mlp_ev_fires(P, e, E.evv[r][e], v)) fired = e;
+      E.evv[r][e] = v;
+    }
+  }
+  if (fired >= 0) {
+    E.evi[r] = fired;
+    R.result[r] = GBDX_EVENT_OCCURRED;
+    E.tfin[r] = tn;
+    if (P.event_root) {
+      // a boolean condition's root is the end of the step
+      double root = tn;
+      if (P.ev_kind[fired] == GBDX_EV_LINEAR) {
+        double cf[6];
+#pragma unroll
+        for (int n = 0; n < 6; n++) cf[n] = P.ev_coef[6 * fired + n];
+        bool ok = true;
+        root = mlp_ev_root<SOLVER, S>(P, ES, r, cf, D < 4 ? D : 4, tp, tn, ok);
+        if (!ok) R.result[r] = GBDX_NONLINEAR_MAX_STEPS;
+      }
+      const double span = tn - tp;
+      E.tfin[r] = root;
+      E.tsave[r] = root;
+      E.thfin[r] = float(span == 0.0 ? 0.0 : (root - tp) / span);
+    }
+  }
+}
+
 // ---------------------------------------------------------------------------
 // The kernel.
 // ---------------------------------------------------------------------------
@@ -798,6 +830,8 @@ __global__ void __launch_bounds__(256) mlp_fused_kernel(SolveParams P) {
   RowState<M> &R = sm.rows;
   RowEvents<M> *EV =
       XO ? reinterpret_cast<RowEvents<M> *>(smem_raw + mlp_events_offset<Sm>()) : nullptr;
+  [[maybe_unused]] RowEventStep<M, 8> *ESP =
+      XO ? reinterpret_cast<RowEventStep<M, 8> *>(EV + 1) : nullptr;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const float *W = P.mlp;
 
@@ -884,13 +918,13 @@ __global__ void __launch_bounds__(256) mlp_fused_kernel(SolveParams P) {
       if (ev_steady) {
         const int fresh = tid < M && live && R.nsteps[tid] == 0;
         if (__syncthreads_or(fresh)) {
-          steady_partials<SH>(*EV, F, Y0, warp, lane);
+          steady_partials<SH>(*ESP, F, Y0, warp, lane);
           __syncthreads();
           if (fresh) {
 #pragma unroll
             for (int e = 0; e < GBDX_MAX_EVENTS; e++) {
               if (e < P.n_event && P.ev_kind[e] == GBDX_EV_STEADY) {
-                const double v = steady_value<SH>(P, *EV, tid, e);
+                const double v = steady_value<D, SH::NT>(P, *ESP, tid, e);
                 EV->evv[tid][e] = v;
                 if (EV->evi[tid] < 0 && v != 0.0) EV->evi[tid] = e;
               }
@@ -969,14 +1003,14 @@ __global__ void __launch_bounds__(256) mlp_fused_kernel(SolveParams P) {
           }
           part += __shfl_xor_sync(0xffffffffu, part, 1);
           part += __shfl_xor_sync(0xffffffffu, part, 2);
-          if ((lane & 3) == 0) R.part[row][(warp * SH::TPW + j) % SH::NT] = part;
+          if ((lane & 3) == 0) sm.part[row][(warp * SH::TPW + j) % SH::NT] = part;
         }
       }
       __syncthreads();
       if (tid < M && live) {
         float a = 0.f;
 #pragma unroll
-        for (int n = 0; n < SH::NT; n++) a += R.part[tid][n];
+        for (int n = 0; n < SH::NT; n++) a += sm.part[tid][n];
         R.acc[tid] = a;
       }
     }
@@ -990,6 +1024,7 @@ __global__ void __launch_bounds__(256) mlp_fused_kernel(SolveParams P) {
     if constexpr (XO) {
     if (P.n_event > 0) {
       RowEvents<M> &E = *EV;
+      RowEventStep<M, 8> &ES = *ESP;
       if constexpr (!TB::FSAL) {
         // f(y1) for a steady-state condition (FSAL solvers have it in F)
         if (ev_steady && __syncthreads_or(tid < M && live && R.keep[tid])) {
@@ -1003,58 +1038,18 @@ __global__ void __launch_bounds__(256) mlp_fused_kernel(SolveParams P) {
         int row, col;
         elem_rc<SH>(e, warp, lane, row, col);
         if (col < 4 && R.live[row] && R.keep[row]) {
-          E.ey0[row][col] = Y0[e];
-          E.ey1[row][col] = Y1[e];
+          ES.ey0[row][col] = Y0[e];
+          ES.ey1[row][col] = Y1[e];
 #pragma unroll
-          for (int j = 0; j < S; j++) E.ek[row][j][col] = K[j][e];
+          for (int j = 0; j < S; j++) ES.ek[row][j][col] = K[j][e];
         }
       }
-      if (ev_steady) steady_partials<SH>(E, F, Y1, warp, lane);
+      if (ev_steady) steady_partials<SH>(ES, F, Y1, warp, lane);
       __syncthreads();
       if (tid < M) {
         E.tsave[tid] = R.tn_old[tid];
         if (live && R.keep[tid]) {
-          const double tn = R.tn_old[tid], tp = R.tp_old[tid];
-          int fired = -1;
-#pragma unroll
-          for (int e = 0; e < GBDX_MAX_EVENTS; e++) {
-            if (e < P.n_event) {
-              double v;
-              if (P.ev_kind[e] == GBDX_EV_STEADY) {
-                v = steady_value<SH>(P, E, tid, e);
-              } else {
-                v = 0.0;
-                for (int n = 0; n < (D < 4 ? D : 4); n++)
-                  v += P.ev_coef[6 * e + n] * double(E.ey1[tid][n]);
-                v += P.ev_coef[6 * e + 4] * tn;
-                v += P.ev_coef[6 * e + 5];
-                if (P.ev_kind[e] == GBDX_EV_LINEAR_BOOL) v = v > 0 ? 1.0 : 0.0;
-              }
-              if (fired < 0 && mlp_ev_fires(P, e, E.evv[tid][e], v)) fired = e;
-              E.evv[tid][e] = v;
-            }
-          }
-          if (fired >= 0) {
-            E.evi[tid] = fired;
-            R.result[tid] = GBDX_EVENT_OCCURRED;
-            E.tfin[tid] = tn;
-            if (P.event_root) {
-              // a boolean condition's root is the end of the step
-              double root = tn;
-              if (P.ev_kind[fired] == GBDX_EV_LINEAR) {
-                double cf[6];
-#pragma unroll
-                for (int n = 0; n < 6; n++) cf[n] = P.ev_coef[6 * fired + n];
-                bool ok = true;
-                root = mlp_ev_root<SOLVER, S>(P, E, tid, cf, D < 4 ? D : 4, tp, tn, ok);
-                if (!ok) R.result[tid] = GBDX_NONLINEAR_MAX_STEPS;
-              }
-              const double span = tn - tp;
-              E.tfin[tid] = root;
-              E.tsave[tid] = root;
-              E.thfin[tid] = float(span == 0.0 ? 0.0 : (root - tp) / span);
-            }
-          }
+          row_events<SOLVER, S, D, SH::NT>(R, E, ES, tid, P);
         }
       }
       __syncthreads();

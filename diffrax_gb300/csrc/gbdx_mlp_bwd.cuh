@@ -88,8 +88,7 @@ struct BwdSmem;
 // which are dead once dW2 has been accumulated.
 template <class SH, bool SDE>
 struct BwdSmem<SH, false, SDE> {
-  static_assert(SH::NP == 3 && !SH::GFRAG,
-                "three-piece operands, weights in shared memory");
+  static_assert(SH::NP == 3, "three-piece operands");
   MlpSmem<SH, false, SDE> f;  // weights, biases, X, A1, A2 (forward recompute)
   __nv_bfloat16 G3[SH::M][SH::PD], G3l[SH::M][SH::PD], G3l2[SH::M][SH::PD];
   __nv_bfloat16 Gs[SDE ? SH::M : 1][SH::PD], Gsl[SDE ? SH::M : 1][SH::PD],

@@ -13,7 +13,9 @@ namespace gbdx {
 template <int D, int H, bool PRECISE, bool SDE, bool XO>
 constexpr size_t mlp_smem_bytes() {
   using Sm = typename MlpField<MlpShape<D, H>, PRECISE, SDE>::Sm;
-  return XO ? mlp_events_offset<Sm>() + sizeof(RowEvents<MlpShape<D, H>::M>) : sizeof(Sm);
+  return XO ? mlp_events_offset<Sm>() + sizeof(RowEvents<MlpShape<D, H>::M>) +
+                  sizeof(RowEventStep<MlpShape<D, H>::M, 8>)
+            : sizeof(Sm);
 }
 
 template <int SOLVER, int D, int H, bool PRECISE, bool SDE, bool XO>
@@ -69,8 +71,9 @@ OdeEntry mlp_entry(int solver, bool precise, bool sde) {
       return OdeEntry{nullptr, nullptr};
     }
   }
+  // (BF16 ODEs: the feature-major form, gbdx_mlp_fm.cuh)
   return precise ? mlp_entry_for_solver<D, H, true, false, XO>(solver)
-                 : mlp_entry_for_solver<D, H, false, false, XO>(solver);
+                 : OdeEntry{nullptr, nullptr};
 }
 
 }  // namespace gbdx

@@ -15,6 +15,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "gbdx_f2.cuh"
+
 namespace gbdx {
 namespace tc {
 
@@ -47,6 +49,15 @@ __host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N) {
          | (1u << 10)                    // B format: BF16
          | (uint32_t(N >> 3) << 17)      // N / 8
          | (uint32_t(M >> 4) << 24);     // M / 16
+}
+
+// The same with MN-major operands: a set flag means the operand's rows (M or N)
+// run contiguously in shared memory and K across them, so 8 rows x 8 k of BF16
+// are one 128-byte core matrix of 16-byte runs along the rows; the descriptor's
+// leading byte offset is then the stride between groups of 8 k and its stride
+// byte offset that between groups of 8 rows.
+__host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N, bool a_mn, bool b_mn) {
+  return idesc_bf16_f32(M, N) | (uint32_t(a_mn) << 15) | (uint32_t(b_mn) << 16);
 }
 
 // TMEM allocation of `ncols` columns (a power of two >= 32) by one whole warp;
@@ -105,6 +116,17 @@ __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a_desc, uint6
       :: "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
 
+// The same with A in tensor memory: lane m holds row m, each 32-bit column two
+// consecutive k.
+__device__ __forceinline__ void mma_bf16_ta(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc,
+                                            uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      :: "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+}
+
 // Arrives on `bar` once every MMA this thread issued so far has completed.
 __device__ __forceinline__ void mma_commit(uint64_t *bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
@@ -130,6 +152,59 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
                :: "memory");
 #pragma unroll
   for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
+}
+
+// Four 32-bit columns of this thread's TMEM lane (tmem_st_wait before use).
+__device__ __forceinline__ void tmem_st4(uint32_t taddr, const uint32_t (&v)[4]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};"
+               :: "r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() {
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+
+// The sums of three runs of 8 (or 4) FP32 columns of this thread's TMEM lane,
+// `stride` columns apart: the products of an operand's three BF16 pieces, the
+// smallest first.
+__device__ __forceinline__ void tmem_sum3(uint32_t taddr, uint32_t stride, F2 (&v)[4]) {
+  uint32_t r[24];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%24];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%8, %9, %10, %11, %12, %13, %14, %15}, [%25];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%16, %17, %18, %19, %20, %21, %22, %23}, [%26];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=&r"(r[0]), "=&r"(r[1]), "=&r"(r[2]), "=&r"(r[3]), "=&r"(r[4]), "=&r"(r[5]),
+        "=&r"(r[6]), "=&r"(r[7]), "=&r"(r[8]), "=&r"(r[9]), "=&r"(r[10]), "=&r"(r[11]),
+        "=&r"(r[12]), "=&r"(r[13]), "=&r"(r[14]), "=&r"(r[15]), "=&r"(r[16]), "=&r"(r[17]),
+        "=&r"(r[18]), "=&r"(r[19]), "=&r"(r[20]), "=&r"(r[21]), "=&r"(r[22]), "=&r"(r[23])
+      : "r"(taddr), "r"(taddr + stride), "r"(taddr + 2 * stride)
+      : "memory");
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    auto pair = [&](int j) {
+      return f2_pack(__uint_as_float(r[j + 2 * i]), __uint_as_float(r[j + 2 * i + 1]));
+    };
+    v[i] = f2_add(f2_add(pair(16), pair(8)), pair(0));
+  }
+}
+__device__ __forceinline__ void tmem_sum3(uint32_t taddr, uint32_t stride, F2 (&v)[2]) {
+  uint32_t r[12];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%12];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%4, %5, %6, %7}, [%13];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%8, %9, %10, %11}, [%14];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=&r"(r[0]), "=&r"(r[1]), "=&r"(r[2]), "=&r"(r[3]), "=&r"(r[4]), "=&r"(r[5]),
+        "=&r"(r[6]), "=&r"(r[7]), "=&r"(r[8]), "=&r"(r[9]), "=&r"(r[10]), "=&r"(r[11])
+      : "r"(taddr), "r"(taddr + stride), "r"(taddr + 2 * stride)
+      : "memory");
+#pragma unroll
+  for (int i = 0; i < 2; i++) {
+    auto pair = [&](int j) {
+      return f2_pack(__uint_as_float(r[j + 2 * i]), __uint_as_float(r[j + 2 * i + 1]));
+    };
+    v[i] = f2_add(f2_add(pair(8), pair(4)), pair(0));
+  }
 }
 
 }  // namespace tc

@@ -69,10 +69,10 @@ enum gbdx_field {
 enum gbdx_diffusion { GBDX_DIFF_NONE = 0, GBDX_DIFF_OU = 1, GBDX_DIFF_TANH_DIAG = 2 };
 enum gbdx_dtype { GBDX_F32 = 0, GBDX_F64 = 1 };
 /* Kernel family: PLAIN is one trajectory per thread launched once per
- * trajectory; FUSED is the persistent work-stealing integrator; TC is the
- * MLP-field forward on the fifth-generation tensor cores (tcgen05.mma with the
- * accumulators and the Runge--Kutta stages in tensor memory; 64 -> 128 -> 128
- * -> 64 fields, Tsit5, BF16 products, forward solves). */
+ * trajectory; FUSED is the persistent work-stealing integrator (the MLP ODE
+ * fields' BF16 forward on the fifth-generation tensor cores); TC asks for that
+ * tensor-core forward by name (64 -> 128 -> 128 -> 64 fields, Tsit5 or Dopri5,
+ * BF16 products, forward solves). */
 enum gbdx_kernel {
   GBDX_KERNEL_AUTO = 0,
   GBDX_KERNEL_PLAIN = 1,
