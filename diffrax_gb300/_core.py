@@ -564,7 +564,9 @@ class AbstractAdjoint:
 @dataclasses.dataclass(frozen=True)
 class RecursiveCheckpointAdjoint(AbstractAdjoint):
     """diffrax/_adjoint.py:179-312.  `checkpoints` bounds the per-trajectory
-    checkpoint slots; None means ceil(log2(max_steps)) slots as the reference."""
+    checkpoint slots; None means 128 (the reference: ceil(log2(max_steps))): longer
+    checkpoint segments would take more memory in recomputed states than the slots
+    save, and a second pass over the steps."""
     checkpoints: Optional[int] = None
 
 

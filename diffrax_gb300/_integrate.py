@@ -154,7 +154,7 @@ def lower(terms, solver, stepsize_controller, saveat: SaveAt, *, dim: int, dtype
     if isinstance(adjoint, RecursiveCheckpointAdjoint):
         cp = adjoint.checkpoints
         if cp is None:
-            cp = max(1, math.ceil(math.log2(max(int(max_steps), 2))))
+            cp = min(128, max(2, int(max_steps) // 2 * 2))
         f.update(adjoint=1, checkpoints=int(cp))
     elif isinstance(adjoint, BacksolveAdjoint):
         f.update(adjoint=2)

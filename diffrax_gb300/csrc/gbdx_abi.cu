@@ -629,10 +629,15 @@ int gbdx_problem_create(const gbdx_problem_desc *desc, gbdx_problem **out) {
     p->mlp = true;
     p->rows_per_cta = H >= 256 ? 16 : 32;
     if (d.adjoint == GBDX_ADJ_RECURSIVE) {
-      if (D == 64 && H == 128) p->bwd = gbdx::find_mlp_bwd_entry_d64h128(d.solver, precise, sde);
+      if (D == 64 && H == 128)
+        p->bwd = precise ? gbdx::find_mlp_bwd_entry_d64h128(d.solver, sde)
+                 : sde   ? gbdx::BwdEntry{nullptr, nullptr}
+                         : gbdx::find_mlp_fm_bwd_entry_d64h128(d.solver);
       // (width 256 does not fit the backward's weights and operands in
       // shared memory; that shape is differentiated by BacksolveAdjoint)
-      if (D == 32 && H == 64) p->bwd = gbdx::find_mlp_bwd_entry_d32h64(d.solver, precise, sde);
+      if (D == 32 && H == 64)
+        p->bwd = precise ? gbdx::find_mlp_bwd_entry_d32h64(d.solver, sde)
+                         : gbdx::find_mlp_fm_bwd_entry_d32h64(d.solver, sde);
       if (!p->bwd.launch) {
         delete p;
         return fail(GBDX_ERR_UNSUPPORTED, "no backward kernel for this MLP problem");
@@ -1097,8 +1102,8 @@ int gbdx_solve_bwd(const gbdx_problem *problem, int64_t batch, const double *t0,
   else if (problem->d.mlp_precision == GBDX_MLP_FP32)
     e = gbdx::launch_reduce_partials(Q.part_sum, Q.part_comp, batch > 0 ? L.n_cta : 0, np,
                                      static_cast<float *>(grad_params), s);
-  else  // the tensor-core mode keeps the weight blocks in fragment order
-    e = gbdx::launch_reduce_partials_frag(
+  else  // the tensor-core mode has a layout of its own
+    e = gbdx::launch_reduce_partials_fm(
         Q.part_sum, Q.part_comp, batch > 0 ? L.n_cta : 0, problem->d.dim,
         problem->d.mlp_widths[1], problem->d.diffusion != GBDX_DIFF_NONE,
         static_cast<float *>(grad_params), s);
@@ -1221,7 +1226,7 @@ int gbdx_backsolve_bwd_ex(const gbdx_problem *problem, int64_t batch, const doub
     e = gbdx::launch_reduce_partials(Q.psum, Q.pcomp, batch > 0 ? L.n_cta : 0, np,
                                      static_cast<float *>(grad_params), s);
   else
-    e = gbdx::launch_reduce_partials_frag(Q.psum, Q.pcomp, batch > 0 ? L.n_cta : 0, D, H, 0,
+    e = gbdx::launch_reduce_partials_frag(Q.psum, Q.pcomp, batch > 0 ? L.n_cta : 0, D, H,
                                           static_cast<float *>(grad_params), s);
   if (e != cudaSuccess) return cuda_fail(e, "gradient reduction");
   return bounds_report(P, s, "gbdx_backsolve_bwd");

@@ -63,8 +63,14 @@ struct BwdEntry {
   BwdLaunchFn launch;
   BwdOccFn occupancy;
 };
-BwdEntry find_mlp_bwd_entry_d64h128(int solver, bool precise, bool sde);
-BwdEntry find_mlp_bwd_entry_d32h64(int solver, bool precise, bool sde);
+BwdEntry find_mlp_bwd_entry_d64h128(int solver, bool sde);
+BwdEntry find_mlp_bwd_entry_d32h64(int solver, bool sde);
+// (above: FP32 products.)  The BF16 forms: feature-major on tcgen05.
+BwdEntry find_mlp_fm_bwd_entry_d64h128(int solver);
+BwdEntry find_mlp_fm_bwd_entry_d32h64(int solver, bool sde);
+// The reduction of their partials (their own block layout) to the flat order.
+cudaError_t launch_reduce_partials_fm(const float *psum, const float *pcomp, int n_cta, int D,
+                                      int H, int diffusion, float *out, cudaStream_t s);
 // grad[p] = compensated sum over CTAs of (psum - pcomp)[cta][p]
 cudaError_t launch_reduce_partials(const float *psum, const float *pcomp, int n_cta,
                                    int n_params, float *out, cudaStream_t s);
@@ -90,10 +96,9 @@ BsEntry find_plain_backsolve_entry(int solver, int D, int H);
 cudaError_t launch_frag_prep(const float *W, int ldw, int K, int N, int trans, uint2 *out,
                              cudaStream_t s);
 // The same for partials whose weight blocks are in mma-fragment order (MLP
-// D -> H -> H -> D, then with `diffusion` the neural SDE's D x D diffusion),
-// written to grad in the flat order.
+// D -> H -> H -> D), written to grad in the flat order.
 cudaError_t launch_reduce_partials_frag(const float *psum, const float *pcomp, int n_cta, int D,
-                                        int H, int diffusion, float *out, cudaStream_t s);
+                                        int H, float *out, cudaStream_t s);
 OdeEntry find_mlp_plain_entry(int solver, int D, int H, bool sde);
 // The plain (one trajectory per thread) RecursiveCheckpointAdjoint backward:
 // full tape, per-trajectory parameter cotangents dP [n_params][batch].

@@ -78,28 +78,8 @@ struct BwdRows {
 enum { kModeBwd = 0, kModeFwd = 1 };
 enum { kLoadNone = 0, kLoadCheckpoint = 1, kLoadScratch = 2 };
 
-template <class SH, bool PRECISE, bool SDE>
-struct BwdSmem;
-
-// The cotangents are held as three BF16 pieces like the forward's
-// activations (24 significant bits), so the gradient keeps the accuracy of an
-// FP32 evaluation with the same BF16 weights.  The layer-0 cotangent G1 is
-// written into the storage of the layer-1 activations A2 (all three pieces),
-// which are dead once dW2 has been accumulated.
 template <class SH, bool SDE>
-struct BwdSmem<SH, false, SDE> {
-  static_assert(SH::NP == 3, "three-piece operands");
-  MlpSmem<SH, false, SDE> f;  // weights, biases, X, A1, A2 (forward recompute)
-  __nv_bfloat16 G3[SH::M][SH::PD], G3l[SH::M][SH::PD], G3l2[SH::M][SH::PD];
-  __nv_bfloat16 Gs[SDE ? SH::M : 1][SH::PD], Gsl[SDE ? SH::M : 1][SH::PD],
-      Gsl2[SDE ? SH::M : 1][SH::PD];
-  __nv_bfloat16 G2[SH::M][SH::PH], G2l[SH::M][SH::PH], G2l2[SH::M][SH::PH];
-  float db0[SH::H], db1[SH::H], db2[SH::D], dbs[SH::D];
-  BwdRows<SH::M> rows;
-};
-
-template <class SH, bool SDE>
-struct BwdSmem<SH, true, SDE> {
+struct BwdSmem {
   MlpSmem<SH, true, SDE> f;
   float G3[SH::M][SH::D + 1];
   float Gs[SDE ? SH::M : 1][SH::D + 1];
@@ -109,62 +89,9 @@ struct BwdSmem<SH, true, SDE> {
   BwdRows<SH::M> rows;
 };
 
-// dW[o][n] (the [O][N] block at offset `off`) += G^T S over the tile's rows,
-// with G and S held as three BF16 pieces each (warp_tile_gemm_tt3),
-// accumulated into this CTA's Kahan partials.  The partials of a weight block
-// are in mma-fragment order: m16n8 tile t = (o / 16) (N / 8) + n / 8 holds its
-// 128 values at off + 128 t + 4 lane + q, q indexing the accumulator elements
-// (g, 2c), (g, 2c + 1), (g + 8, 2c), (g + 8, 2c + 1), so a lane's four values
-// are one 16-byte load and store (the final reduction restores the flat
-// order).
-template <class SH, int O, int N>
-__device__ __forceinline__ void dw_tiles(const __nv_bfloat16 *const (&G)[3], int ldg,
-                                         const __nv_bfloat16 *const (&S)[3], int lds, int off,
-                                         float *psum, float *pcomp, int warp, int lane) {
-  constexpr int TILES = (O / 16) * (N / 8);
-  static_assert(TILES % SH::WARPS == 0, "weight-gradient tile split");
-  constexpr int T = TILES / SH::WARPS;
-  constexpr int CH = T < 8 ? T : 8;
-  static_assert((N / 8) % CH == 0 && T % CH == 0, "weight-gradient chunk split");
-  const int g = lane >> 2, c = lane & 3;
-#pragma unroll 1
-  for (int ch = 0; ch < T / CH; ch++) {
-    const int t = warp * T + ch * CH;
-    const int ot = t / (N / 8), nt0 = t % (N / 8);
-    // the partials this chunk updates are loaded before its products, so the
-    // L2 latency overlaps the tensor-core work
-    float4 ps[CH], pc[CH];
-#pragma unroll
-    for (int j = 0; j < CH; j++) {
-      const int p = off + (t + j) * 128 + lane * 4;
-      ps[j] = *reinterpret_cast<const float4 *>(psum + p);
-      pc[j] = *reinterpret_cast<const float4 *>(pcomp + p);
-    }
-    float acc[CH][4];
-#pragma unroll
-    for (int j = 0; j < CH; j++) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
-    warp_tile_gemm_tt3<SH::M, CH>(acc, G, ldg, ot * 16, S, lds, nt0 * 8, lane);
-#pragma unroll
-    for (int j = 0; j < CH; j++) {
-      float sv[4] = {ps[j].x, ps[j].y, ps[j].z, ps[j].w};
-      float cv[4] = {pc[j].x, pc[j].y, pc[j].z, pc[j].w};
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-        const float y = acc[j][q] - cv[q];
-        const float tq = sv[q] + y;
-        cv[q] = (tq - sv[q]) - y;
-        sv[q] = tq;
-      }
-      const int p = off + (t + j) * 128 + lane * 4;
-      *reinterpret_cast<float4 *>(psum + p) = make_float4(sv[0], sv[1], sv[2], sv[3]);
-      *reinterpret_cast<float4 *>(pcomp + p) = make_float4(cv[0], cv[1], cv[2], cv[3]);
-    }
-  }
-}
-
-template <class SH, bool PRECISE, bool SDE>
+template <class SH, bool SDE>
 struct MlpVjp {
-  using Sm = BwdSmem<SH, PRECISE, SDE>;
+  using Sm = BwdSmem<SH, SDE>;
   static constexpr int D = SH::D, H = SH::H, M = SH::M, NE = SH::NE;
 
   // Given the forward recompute of one stage (X, A1, A2 in smem; sig in
@@ -181,178 +108,71 @@ struct MlpVjp {
       elem_rc<SH>(e, warp, lane, row, col);
       // sigma = 0.1 tanh(z): d sigma / dz = 0.1 (1 - (sigma / 0.1)^2)
       const float gz = SDE ? Gsr[e] * 0.1f * (1.f - 100.f * sig[e] * sig[e]) : 0.f;
-      if constexpr (PRECISE) {
-        sm.G3[row][col] = G3r[e];
-        if constexpr (SDE) sm.Gs[row][col] = gz;
-      } else {
-        if ((e & 1) == 0)
-          store_split3x2(G3r[e], G3r[e + 1], &sm.G3[row][col], &sm.G3l[row][col],
-                         &sm.G3l2[row][col]);
-        if constexpr (SDE) split_store3(gz, &sm.Gs[row][col], &sm.Gsl[row][col], &sm.Gsl2[row][col]);
-      }
+      sm.G3[row][col] = G3r[e];
+      if constexpr (SDE) sm.Gs[row][col] = gz;
       if (G3r[e] != 0.f) atomicAdd(&sm.db2[col], G3r[e]);
       if (SDE && gz != 0.f) atomicAdd(&sm.dbs[col], gz);
     }
     __syncthreads();
-    if constexpr (PRECISE) {
-      const float *W0 = P + SH::OW0, *W1 = P + SH::OW1, *W2 = P + SH::OW2, *Ws = P + SH::OWS;
-      // 2. G2 = (G3 W2) * (1 - A2^2); dW2 += G3^T A2
-      for (int i = tid; i < M * H; i += SH::THREADS) {
-        const int r = i / H, hh = i % H;
-        float a = 0.f;
-        for (int d = 0; d < D; d++) a = fmaf(sm.G3[r][d], __ldg(W2 + d * H + hh), a);
-        const float ah = sm.f.A2[r][hh];
-        const float v = a * (1.f - ah * ah);
-        sm.G2[r][hh] = v;
-        if (v != 0.f) atomicAdd(&sm.db1[hh], v);
-      }
-      for (int i = tid; i < D * H; i += SH::THREADS) {
-        const int d = i / H, hh = i % H;
-        float a = 0.f;
-        for (int r = 0; r < M; r++) a = fmaf(sm.G3[r][d], sm.f.A2[r][hh], a);
-        kahan_add(psum + SH::OW2 + i, pcomp + SH::OW2 + i, a);
-      }
-      __syncthreads();
-      // 3. G1 = (G2 W1) * (1 - A1^2); dW1 += G2^T A1
-      for (int i = tid; i < M * H; i += SH::THREADS) {
-        const int r = i / H, hh = i % H;
-        float a = 0.f;
-        for (int o = 0; o < H; o++) a = fmaf(sm.G2[r][o], __ldg(W1 + o * H + hh), a);
-        const float ah = sm.f.A1[r][hh];
-        const float v = a * (1.f - ah * ah);
-        sm.G1[r][hh] = v;
-        if (v != 0.f) atomicAdd(&sm.db0[hh], v);
-      }
-      for (int i = tid; i < H * H; i += SH::THREADS) {
-        const int o = i / H, hh = i % H;
-        float a = 0.f;
-        for (int r = 0; r < M; r++) a = fmaf(sm.G2[r][o], sm.f.A1[r][hh], a);
-        kahan_add(psum + SH::OW1 + i, pcomp + SH::OW1 + i, a);
-      }
-      __syncthreads();
-      // 4. gY = G1 W0 (+ Gs Ws); dW0 += G1^T X (dWs += Gs^T X)
+    const float *W0 = P + SH::OW0, *W1 = P + SH::OW1, *W2 = P + SH::OW2, *Ws = P + SH::OWS;
+    // 2. G2 = (G3 W2) * (1 - A2^2); dW2 += G3^T A2
+    for (int i = tid; i < M * H; i += SH::THREADS) {
+      const int r = i / H, hh = i % H;
+      float a = 0.f;
+      for (int d = 0; d < D; d++) a = fmaf(sm.G3[r][d], __ldg(W2 + d * H + hh), a);
+      const float ah = sm.f.A2[r][hh];
+      const float v = a * (1.f - ah * ah);
+      sm.G2[r][hh] = v;
+      if (v != 0.f) atomicAdd(&sm.db1[hh], v);
+    }
+    for (int i = tid; i < D * H; i += SH::THREADS) {
+      const int d = i / H, hh = i % H;
+      float a = 0.f;
+      for (int r = 0; r < M; r++) a = fmaf(sm.G3[r][d], sm.f.A2[r][hh], a);
+      kahan_add(psum + SH::OW2 + i, pcomp + SH::OW2 + i, a);
+    }
+    __syncthreads();
+    // 3. G1 = (G2 W1) * (1 - A1^2); dW1 += G2^T A1
+    for (int i = tid; i < M * H; i += SH::THREADS) {
+      const int r = i / H, hh = i % H;
+      float a = 0.f;
+      for (int o = 0; o < H; o++) a = fmaf(sm.G2[r][o], __ldg(W1 + o * H + hh), a);
+      const float ah = sm.f.A1[r][hh];
+      const float v = a * (1.f - ah * ah);
+      sm.G1[r][hh] = v;
+      if (v != 0.f) atomicAdd(&sm.db0[hh], v);
+    }
+    for (int i = tid; i < H * H; i += SH::THREADS) {
+      const int o = i / H, hh = i % H;
+      float a = 0.f;
+      for (int r = 0; r < M; r++) a = fmaf(sm.G2[r][o], sm.f.A1[r][hh], a);
+      kahan_add(psum + SH::OW1 + i, pcomp + SH::OW1 + i, a);
+    }
+    __syncthreads();
+    // 4. gY = G1 W0 (+ Gs Ws); dW0 += G1^T X (dWs += Gs^T X)
 #pragma unroll
-      for (int e = 0; e < NE; e++) {
-        int row, col;
-        elem_rc<SH>(e, warp, lane, row, col);
-        float a = 0.f;
-        for (int o = 0; o < H; o++) a = fmaf(sm.G1[row][o], __ldg(W0 + o * D + col), a);
-        if constexpr (SDE)
-          for (int o = 0; o < D; o++) a = fmaf(sm.Gs[row][o], __ldg(Ws + o * D + col), a);
-        gY[e] = a;
-      }
-      for (int i = tid; i < H * D; i += SH::THREADS) {
+    for (int e = 0; e < NE; e++) {
+      int row, col;
+      elem_rc<SH>(e, warp, lane, row, col);
+      float a = 0.f;
+      for (int o = 0; o < H; o++) a = fmaf(sm.G1[row][o], __ldg(W0 + o * D + col), a);
+      if constexpr (SDE)
+        for (int o = 0; o < D; o++) a = fmaf(sm.Gs[row][o], __ldg(Ws + o * D + col), a);
+      gY[e] = a;
+    }
+    for (int i = tid; i < H * D; i += SH::THREADS) {
+      const int o = i / D, d = i % D;
+      float a = 0.f;
+      for (int r = 0; r < M; r++) a = fmaf(sm.G1[r][o], sm.f.X[r][d], a);
+      kahan_add(psum + SH::OW0 + i, pcomp + SH::OW0 + i, a);
+    }
+    if constexpr (SDE)
+      for (int i = tid; i < D * D; i += SH::THREADS) {
         const int o = i / D, d = i % D;
         float a = 0.f;
-        for (int r = 0; r < M; r++) a = fmaf(sm.G1[r][o], sm.f.X[r][d], a);
-        kahan_add(psum + SH::OW0 + i, pcomp + SH::OW0 + i, a);
+        for (int r = 0; r < M; r++) a = fmaf(sm.Gs[r][o], sm.f.X[r][d], a);
+        kahan_add(psum + SH::OWS + i, pcomp + SH::OWS + i, a);
       }
-      if constexpr (SDE)
-        for (int i = tid; i < D * D; i += SH::THREADS) {
-          const int o = i / D, d = i % D;
-          float a = 0.f;
-          for (int r = 0; r < M; r++) a = fmaf(sm.Gs[r][o], sm.f.X[r][d], a);
-          kahan_add(psum + SH::OWS + i, pcomp + SH::OWS + i, a);
-        }
-    } else {
-      const int g = lane >> 2, c = lane & 3;
-      const __nv_bfloat16 *const G3p[3] = {&sm.G3[0][0], &sm.G3l[0][0], &sm.G3l2[0][0]};
-      const __nv_bfloat16 *const G2p[3] = {&sm.G2[0][0], &sm.G2l[0][0], &sm.G2l2[0][0]};
-      {  // 2. G2 = (G3 W2) * (1 - A2^2), hidden-tile layout
-        const int t0 = warp * SH::TPWH, mt = t0 / SH::NTH, nt0 = t0 % SH::NTH;
-        float acc[SH::TPWH][4];
-#pragma unroll
-        for (int j = 0; j < SH::TPWH; j++) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
-        warp_tile_gemm_bt3<D, SH::TPWH>(acc, &sm.G3[mt * 16][0], &sm.G3l[mt * 16][0],
-                                        &sm.G3l2[mt * 16][0], SH::PD, &sm.f.W2[0][0], SH::PH,
-                                        nt0 * 8, lane);
-        auto A2 = sm.f.a2();
-        auto A2l = sm.f.a2l();
-        auto A2l2 = sm.f.a2l2();
-#pragma unroll
-        for (int j = 0; j < SH::TPWH; j++)
-#pragma unroll
-          for (int hr = 0; hr < 2; hr++) {
-            const int row = mt * 16 + g + hr * 8, col = (nt0 + j) * 8 + 2 * c;
-            const float a0 = __bfloat162float(A2[row][col]) + __bfloat162float(A2l[row][col]) +
-                             __bfloat162float(A2l2[row][col]);
-            const float a1 = __bfloat162float(A2[row][col + 1]) +
-                             __bfloat162float(A2l[row][col + 1]) +
-                             __bfloat162float(A2l2[row][col + 1]);
-            const float v0 = acc[j][2 * hr] * (1.f - a0 * a0);
-            const float v1 = acc[j][2 * hr + 1] * (1.f - a1 * a1);
-            store_split3x2(v0, v1, &sm.G2[row][col], &sm.G2l[row][col], &sm.G2l2[row][col]);
-            if (v0 != 0.f) atomicAdd(&sm.db1[col], v0);
-            if (v1 != 0.f) atomicAdd(&sm.db1[col + 1], v1);
-          }
-      }
-      {
-        const __nv_bfloat16 *const A2p[3] = {&sm.f.a2()[0][0], &sm.f.a2l()[0][0],
-                                             &sm.f.a2l2()[0][0]};
-        dw_tiles<SH, D, H>(G3p, SH::PD, A2p, SH::PH, SH::OW2, psum, pcomp, warp, lane);
-      }
-      __syncthreads();
-      // A2 is dead from here: G1 (three pieces) takes its storage
-      __nv_bfloat16(*G1)[SH::PH] = sm.f.a2();
-      __nv_bfloat16(*G1l)[SH::PH] = sm.f.a2l();
-      __nv_bfloat16(*G1l2)[SH::PH] = sm.f.a2l2();
-      {  // 3. G1 = (G2 W1) * (1 - A1^2)
-        const int t0 = warp * SH::TPWH, mt = t0 / SH::NTH, nt0 = t0 % SH::NTH;
-        float acc[SH::TPWH][4];
-#pragma unroll
-        for (int j = 0; j < SH::TPWH; j++) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
-        warp_tile_gemm_bt3<H, SH::TPWH>(acc, &sm.G2[mt * 16][0], &sm.G2l[mt * 16][0],
-                                        &sm.G2l2[mt * 16][0], SH::PH, &sm.f.W1[0][0], SH::PH,
-                                        nt0 * 8, lane);
-#pragma unroll
-        for (int j = 0; j < SH::TPWH; j++)
-#pragma unroll
-          for (int hr = 0; hr < 2; hr++) {
-            const int row = mt * 16 + g + hr * 8, col = (nt0 + j) * 8 + 2 * c;
-            const float a0 = __bfloat162float(sm.f.A1[row][col]) +
-                             __bfloat162float(sm.f.A1l[row][col]) +
-                             __bfloat162float(sm.f.A1l2[row][col]);
-            const float a1 = __bfloat162float(sm.f.A1[row][col + 1]) +
-                             __bfloat162float(sm.f.A1l[row][col + 1]) +
-                             __bfloat162float(sm.f.A1l2[row][col + 1]);
-            const float v0 = acc[j][2 * hr] * (1.f - a0 * a0);
-            const float v1 = acc[j][2 * hr + 1] * (1.f - a1 * a1);
-            store_split3x2(v0, v1, &G1[row][col], &G1l[row][col], &G1l2[row][col]);
-            if (v0 != 0.f) atomicAdd(&sm.db0[col], v0);
-            if (v1 != 0.f) atomicAdd(&sm.db0[col + 1], v1);
-          }
-      }
-      {
-        const __nv_bfloat16 *const A1p[3] = {&sm.f.A1[0][0], &sm.f.A1l[0][0],
-                                             &sm.f.A1l2[0][0]};
-        dw_tiles<SH, H, H>(G2p, SH::PH, A1p, SH::PH, SH::OW1, psum, pcomp, warp, lane);
-      }
-      __syncthreads();
-      {  // 4. gY = G1 W0 (+ Gs Ws), owned layout
-        const int t0 = warp * SH::TPW, mt = t0 / SH::NT, nt0 = t0 % SH::NT;
-        float acc[SH::TPW][4];
-#pragma unroll
-        for (int j = 0; j < SH::TPW; j++) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
-        warp_tile_gemm_bt3<H, SH::TPW>(acc, &G1[mt * 16][0], &G1l[mt * 16][0],
-                                       &G1l2[mt * 16][0], SH::PH, &sm.f.W0[0][0], SH::PW0,
-                                       nt0 * 8, lane);
-        if constexpr (SDE)
-          warp_tile_gemm_bt3<D, SH::TPW>(acc, &sm.Gs[mt * 16][0], &sm.Gsl[mt * 16][0],
-                                         &sm.Gsl2[mt * 16][0], SH::PD, &sm.f.Ws[0][0], SH::PD,
-                                         nt0 * 8, lane);
-#pragma unroll
-        for (int e = 0; e < NE; e++) gY[e] = acc[e >> 2][e & 3];
-      }
-      const __nv_bfloat16 *const Xp[3] = {&sm.f.X[0][0], &sm.f.Xl[0][0], &sm.f.Xl2[0][0]};
-      {
-        const __nv_bfloat16 *const G1p[3] = {&G1[0][0], &G1l[0][0], &G1l2[0][0]};
-        dw_tiles<SH, H, D>(G1p, SH::PH, Xp, SH::PD, SH::OW0, psum, pcomp, warp, lane);
-      }
-      if constexpr (SDE) {
-        const __nv_bfloat16 *const Gsp[3] = {&sm.Gs[0][0], &sm.Gsl[0][0], &sm.Gsl2[0][0]};
-        dw_tiles<SH, D, D>(Gsp, SH::PD, Xp, SH::PD, SH::OWS, psum, pcomp, warp, lane);
-      }
-    }
   }
 };
 
@@ -400,11 +220,11 @@ __device__ void bwd_row_init(BwdRows<SH::M> &R, int r, int64_t i, const SolvePar
   }
 }
 
-template <int SOLVER, int D, int H, bool PRECISE, bool SDE>
+template <int SOLVER, int D, int H, bool SDE>
 __global__ void __launch_bounds__(256) mlp_bwd_kernel(SolveParams P, BwdParams Q) {
   using SH = MlpShape<D, H>;
-  using FLD = MlpField<SH, PRECISE, SDE>;
-  using VJP = MlpVjp<SH, PRECISE, SDE>;
+  using FLD = MlpField<SH, true, SDE>;
+  using VJP = MlpVjp<SH, SDE>;
   using Sm = typename VJP::Sm;
   using TB = Tab<SOLVER>;
   constexpr int S = TB::S, NE = SH::NE, M = SH::M;

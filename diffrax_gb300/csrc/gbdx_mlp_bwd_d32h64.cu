@@ -3,7 +3,7 @@
 #include "gbdx_mlp_bwd_impl.cuh"
 
 namespace gbdx {
-BwdEntry find_mlp_bwd_entry_d32h64(int solver, bool precise, bool sde) {
-  return mlp_bwd_entry<32, 64, true>(solver, precise, sde);
+BwdEntry find_mlp_bwd_entry_d32h64(int solver, bool sde) {
+  return mlp_bwd_entry<32, 64, true>(solver, sde);
 }
 }  // namespace gbdx

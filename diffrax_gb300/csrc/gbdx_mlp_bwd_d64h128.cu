@@ -3,7 +3,7 @@
 #include "gbdx_mlp_bwd_impl.cuh"
 
 namespace gbdx {
-BwdEntry find_mlp_bwd_entry_d64h128(int solver, bool precise, bool sde) {
-  return mlp_bwd_entry<64, 128, false>(solver, precise, sde);
+BwdEntry find_mlp_bwd_entry_d64h128(int solver, bool sde) {
+  return mlp_bwd_entry<64, 128, false>(solver, sde);
 }
 }  // namespace gbdx

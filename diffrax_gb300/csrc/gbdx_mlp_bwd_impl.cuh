@@ -1,4 +1,5 @@
-// gbdx_mlp_bwd_impl.cuh -- launchers of the MLP-field backward for one shape.
+// gbdx_mlp_bwd_impl.cuh -- launchers of the MLP-field backward (FP32 products) for
+// one shape.
 #pragma once
 
 #include "gbdx_launch.h"
@@ -6,10 +7,10 @@
 
 namespace gbdx {
 
-template <int SOLVER, int D, int H, bool PRECISE, bool SDE>
+template <int SOLVER, int D, int H, bool SDE>
 cudaError_t launch_mlp_bwd(const SolveParams &P, const BwdParams &Q, int grid, cudaStream_t s) {
-  using Sm = typename MlpVjp<MlpShape<D, H>, PRECISE, SDE>::Sm;
-  auto k = mlp_bwd_kernel<SOLVER, D, H, PRECISE, SDE>;
+  using Sm = typename MlpVjp<MlpShape<D, H>, SDE>::Sm;
+  auto k = mlp_bwd_kernel<SOLVER, D, H, SDE>;
   cudaError_t e =
       cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Sm));
   if (e != cudaSuccess) return e;
@@ -18,20 +19,20 @@ cudaError_t launch_mlp_bwd(const SolveParams &P, const BwdParams &Q, int grid, c
   return cudaGetLastError();
 }
 
-template <int SOLVER, int D, int H, bool PRECISE, bool SDE>
+template <int SOLVER, int D, int H, bool SDE>
 cudaError_t occupancy_mlp_bwd(int *ctas) {
-  using Sm = typename MlpVjp<MlpShape<D, H>, PRECISE, SDE>::Sm;
-  auto k = mlp_bwd_kernel<SOLVER, D, H, PRECISE, SDE>;
+  using Sm = typename MlpVjp<MlpShape<D, H>, SDE>::Sm;
+  auto k = mlp_bwd_kernel<SOLVER, D, H, SDE>;
   cudaError_t e =
       cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Sm));
   if (e != cudaSuccess) return e;
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas, k, 256, sizeof(Sm));
 }
 
-template <int D, int H, bool PRECISE, bool SDE>
+template <int D, int H, bool SDE>
 BwdEntry mlp_bwd_entry_for_solver(int solver) {
 #define GBDX_BWD_ENTRY(S) \
-  BwdEntry { &launch_mlp_bwd<S, D, H, PRECISE, SDE>, &occupancy_mlp_bwd<S, D, H, PRECISE, SDE> }
+  BwdEntry { &launch_mlp_bwd<S, D, H, SDE>, &occupancy_mlp_bwd<S, D, H, SDE> }
   switch (solver) {
     case GBDX_EULER: return GBDX_BWD_ENTRY(GBDX_EULER);
     case GBDX_HEUN: return GBDX_BWD_ENTRY(GBDX_HEUN);
@@ -47,18 +48,17 @@ BwdEntry mlp_bwd_entry_for_solver(int solver) {
   return BwdEntry{nullptr, nullptr};
 }
 
+// (BF16 products: gbdx_mlp_fm_bwd.cuh)
 template <int D, int H, bool WITH_SDE>
-BwdEntry mlp_bwd_entry(int solver, bool precise, bool sde) {
+BwdEntry mlp_bwd_entry(int solver, bool sde) {
   if (sde) {
     if constexpr (WITH_SDE) {
-      return precise ? mlp_bwd_entry_for_solver<D, H, true, true>(solver)
-                     : mlp_bwd_entry_for_solver<D, H, false, true>(solver);
+      return mlp_bwd_entry_for_solver<D, H, true>(solver);
     } else {
       return BwdEntry{nullptr, nullptr};
     }
   }
-  return precise ? mlp_bwd_entry_for_solver<D, H, true, false>(solver)
-                 : mlp_bwd_entry_for_solver<D, H, false, false>(solver);
+  return mlp_bwd_entry_for_solver<D, H, false>(solver);
 }
 
 }  // namespace gbdx
