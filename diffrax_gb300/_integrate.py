@@ -10,6 +10,7 @@ from __future__ import annotations
 
 import ctypes
 import math
+import threading
 from typing import Any, Optional
 
 import torch
@@ -161,8 +162,13 @@ def lower(terms, solver, stepsize_controller, saveat: SaveAt, *, dim: int, dtype
     return f
 
 
+def _cuda() -> bool:
+    # (once there is a context the query, which reads the environment, is not needed)
+    return torch.cuda.is_initialized() or torch.cuda.is_available()
+
+
 def _device():
-    if not torch.cuda.is_available():
+    if not _cuda():
         raise RuntimeError("diffrax_gb300 needs a CUDA device: there is no CPU path")
     return torch.device("cuda", torch.cuda.current_device())
 
@@ -238,7 +244,7 @@ def _time_arrays(t0, t1, dt0, B, dev):
 
 
 def _capturing() -> bool:
-    return torch.cuda.is_available() and torch.cuda.is_current_stream_capturing()
+    return _cuda() and torch.cuda.is_current_stream_capturing()
 
 
 def _host_checks(t0, t1, dt0, ts, tstride):
@@ -260,12 +266,52 @@ def _host_checks(t0, t1, dt0, ts, tstride):
             raise RuntimeError("saveat.ts must lie between t0 and t1.")
 
 
+class _Status(threading.local):
+    """Where gbdx_solve_status leaves a solve's outcome for this thread: per device
+    32 device bytes of scratch and 16 of page-locked host memory that the kernel
+    writes in place, so an outcome costs one launch and one wait for the stream."""
+
+    def __init__(self):
+        self.buffers = {}
+
+    def read(self, dev, result, low=None, ts=None):
+        """(unsorted, outside, failed, code), include/gbdx.h; waits for the stream."""
+        if dev.index != torch.cuda.current_device():
+            with torch.cuda.device(dev):
+                return self.read(dev, result, low, ts)
+        lib = _lib.load()
+        stream = torch.cuda.current_stream(dev)
+        b = self.buffers.get(dev.index)
+        if b is None:
+            host = torch.zeros(4, dtype=torch.int32, pin_memory=True)
+            scratch = torch.zeros(4, dtype=torch.int64, device=dev)
+            stream.synchronize()
+            b = self.buffers[dev.index] = (host, scratch, host.numpy(),
+                                           _lib.host_device_pointer(host.data_ptr()))
+        host, scratch, view, addr = b
+        out = None if addr is not None else torch.empty(4, dtype=torch.int32, device=dev)
+        n_ts = 0 if ts is None else ts.numel()
+        rc = lib.gbdx_solve_status(
+            result.data_ptr(), result.numel(),
+            low.t0.data_ptr() if n_ts else None, low.t1.data_ptr() if n_ts else None,
+            low.tstride if n_ts else 0, ts.data_ptr() if n_ts else None, n_ts,
+            scratch.data_ptr(), addr if out is None else out.data_ptr(), stream.cuda_stream)
+        _lib.check(rc, "gbdx_solve_status")
+        if out is not None:
+            host.copy_(out)
+        stream.synchronize()
+        return view.tolist()
+
+
+_STATUS = _Status()
+
+
 class Lowered:
     """A lowered, validated solve ready for the C ABI (reused by autograd)."""
 
     def __init__(self, terms, solver, t0, t1, dt0, y0, args, saveat, stepsize_controller,
                  adjoint, max_steps, kernel, block_threads, ctas_per_sm, schedule="auto",
-                 want_grad=False, event=None, throw=True):
+                 want_grad=False, event=None, throw=True, defer_checks=False):
         dev = _device()
         # diffrax/_adjoint.py:623-634: the backward solve of BacksolveAdjoint
         # takes the forward's `throw` unless its kwargs override it
@@ -307,7 +353,16 @@ class Lowered:
         self.drift = drift
         self.problem = _lib.get_problem(self.fields)
         self.t0, self.t1, self.dt0, self.tstride = _time_arrays(t0, t1, dt0, self.B, dev)
-        _host_checks(self.t0, self.t1, self.dt0, ts, self.tstride)
+        # With defer_checks the times in ts are checked with the solve's results
+        # (check()): an invalid time is never or wrongly saved, nothing worse.
+        self.ts_unchecked = ts if defer_checks and n_ts and not _capturing() else None
+        if any(isinstance(x, torch.Tensor) for x in (t0, t1, dt0)):
+            _host_checks(self.t0, self.t1, self.dt0, None if defer_checks else ts, self.tstride)
+        else:
+            if dt0 is not None and (t1 - t0) * dt0 < 0 and not _capturing():
+                raise ValueError("Must have (t1 - t0) * dt0 >= 0")
+            if not defer_checks:
+                _host_checks(self.t0, self.t1, None, ts, self.tstride)
         self.bwd_problem = None
         if backsolve:
             # The backward solve reuses the forward's solver and controller
@@ -354,12 +409,26 @@ class Lowered:
             parts.append(drift.flat_params(self.dtype, dev))
         if self.diffusion is not None and hasattr(self.diffusion, "flat_params"):
             parts.append(self.diffusion.flat_params(self.dtype, dev))
-        self.params = torch.cat(parts).contiguous() if parts else None
+        self.params = parts[0] if len(parts) == 1 else torch.cat(parts) if parts else None
         if self.params is not None and self.params.numel() != self.problem.param_count():
             raise ValueError(f"expected {self.problem.param_count()} field parameters, "
                              f"got {self.params.numel()}")
         self.n_save = self.problem.n_save
         self.device = dev
+
+    def check(self, result, throw):
+        """Raises for what was left to check of the times in ts, then (throw) for a
+        failed trajectory; waits for the solve."""
+        ts, self.ts_unchecked = self.ts_unchecked, None
+        if _capturing() or not (throw or ts is not None):
+            return
+        unsorted, outside, failed, code = _STATUS.read(self.device, result, self, ts)
+        if unsorted:
+            raise RuntimeError("saveat.ts must be increasing or decreasing.")
+        if outside:
+            raise RuntimeError("saveat.ts must lie between t0 and t1.")
+        if throw and failed:
+            _raise_failure(code, failed, result.numel())
 
     def _outputs(self, io):
         """ys, ts, result, stats on the device, None for those `io` gives."""
@@ -648,12 +717,18 @@ def _raise_on_failure(result: torch.Tensor):
     if _capturing():
         return
     # successful and event_occurred are both fine (is_okay, _solution.py:52-54)
-    bad = (result != 0) & (result != int(RESULTS.event_occurred))
-    if bool(bad.any()):
-        code = int(result[bad][0].item())
-        n = int(bad.sum().item())
-        raise RuntimeError(f"{RESULT_MESSAGES.get(RESULTS(code), 'failed')} "
-                           f"({n} of {result.numel()} trajectories failed)")
+    if result.is_cuda:
+        _, _, failed, code = _STATUS.read(result.device, result.contiguous())
+    else:
+        bad = result[(result != 0) & (result != int(RESULTS.event_occurred))]
+        failed, code = bad.numel(), int(bad[0]) if bad.numel() else 0
+    if failed:
+        _raise_failure(code, failed, result.numel())
+
+
+def _raise_failure(code, failed, total):
+    raise RuntimeError(f"{RESULT_MESSAGES.get(RESULTS(code), 'failed')} "
+                       f"({failed} of {total} trajectories failed)")
 
 
 def diffeqsolve(terms, solver, t0, t1, dt0, y0, args=None, *,
@@ -723,7 +798,7 @@ def diffeqsolve(terms, solver, t0, t1, dt0, y0, args=None, *,
         kernel, block_threads, ctas_per_sm = autotune_launch(factory, base.B, base.fields)
     low = Lowered(terms, solver, t0, t1, dt0, y0, args, saveat, stepsize_controller,
                   adjoint, max_steps, kernel, block_threads, ctas_per_sm, schedule,
-                  want_grad=want_grad, event=event, throw=throw)
+                  want_grad=want_grad, event=event, throw=throw, defer_checks=True)
     interp = ev = None
     if saveat.dense or event is not None or resume or keep_state:
         rec = None
@@ -741,6 +816,7 @@ def diffeqsolve(terms, solver, t0, t1, dt0, y0, args=None, *,
         # SaveAt(dense=True) or the states alone save no ys (_integrate.py:1527-1539)
         ys = ts_out = None
     elif getattr(saveat, "fn", None) is not None:
+        low.check(res, False)
         ys = saveat.fn(ts_out, ys, args)
     sol = Solution(t0=t0, t1=t1, ts=ts_out, ys=ys,
                    stats=dict(num_steps=stats[:, 0], num_accepted_steps=stats[:, 1],
@@ -754,6 +830,5 @@ def diffeqsolve(terms, solver, t0, t1, dt0, y0, args=None, *,
     # the lowered solve; after a backward pass under BacksolveAdjoint it holds
     # the backward's RESULTS codes and step counts (bwd_result, bwd_stats)
     sol.lowered = low
-    if throw:
-        _raise_on_failure(res)
+    low.check(res, throw)
     return sol

@@ -98,6 +98,8 @@ def load():
         lib.gbdx_backsolve_bwd_ex.argtypes = [vp, i64, vp, vp, vp, i64, vp, vp, vp, vp, i64,
                                               vp, vp, vp, vp, vp, vp, _c.c_size_t, vp]
         lib.gbdx_backsolve_bwd_ex.restype = i32
+        lib.gbdx_solve_status.argtypes = [vp, i64, vp, vp, i64, vp, i32, vp, vp, vp]
+        lib.gbdx_solve_status.restype = i32
         lib.gbdx_last_error.argtypes = []
         lib.gbdx_last_error.restype = _c.c_char_p
         lib.gbdx_version.restype = i32
@@ -198,8 +200,8 @@ _problem_cache: dict = {}
 
 
 def get_problem(fields: dict) -> Problem:
-    key = tuple(sorted((k, tuple(v) if isinstance(v, (list, tuple)) else v)
-                       for k, v in fields.items()))
+    # (in the order the fields were set: another order is at worst another entry)
+    key = tuple([(k, tuple(v)) if type(v) is list else (k, v) for k, v in fields.items()])
     p = _problem_cache.get(key)
     if p is None:
         p = Problem(fields)

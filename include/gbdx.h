@@ -443,6 +443,19 @@ size_t gbdx_problem_desc_size(void);
  * is not page-locked host memory mapped for the current device. */
 int gbdx_host_device_pointer(const void *host, void **device);
 
+/* A solve's outcome for the host, one kernel on `stream` (is_okay,
+ * diffrax/_solution.py:52-54, and the saveat.ts checks, diffrax/_integrate.py:
+ * 1222-1235): status[0] is 1 when ts is not monotone in some trajectory's direction
+ * of time, [1] when some of it lies outside some trajectory's interval, [2] the
+ * number of trajectories whose result is neither successful nor event_occurred, [3]
+ * the code of the first of them.  result may be NULL (no trajectory failed); ts is
+ * checked when n_ts > 0.  scratch: 32 device bytes, zero before the first call and
+ * left zero, for one call at a time.  status: 4 int32, device memory or page-locked
+ * host memory through its device address. */
+int gbdx_solve_status(const int32_t *result, int64_t batch, const double *t0,
+                      const double *t1, int64_t time_stride, const double *ts, int32_t n_ts,
+                      void *scratch, int32_t *status, void *stream);
+
 /* Library version and the message of the last error on this thread. */
 int gbdx_version(void);
 const char *gbdx_last_error(void);
