@@ -10,6 +10,7 @@
 // and round on the guard bits.
 #pragma once
 
+#include <math.h>
 #include <stdint.h>
 #include <string.h>
 
@@ -94,6 +95,17 @@ GBDX_HD double f64i_from_f32(float f) {
   // bits become the top of the 52
   const uint32_t hi = (u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + (896u << 20));
   return f64i_double((uint64_t(hi) << 32) | uint64_t(u << 29));
+}
+
+// float(a - double(f)) for f the rounding of a to binary32: a's pattern and the widened
+// f's differ by their distance in units of a's last place, also across a power of two.
+GBDX_HD float f64i_rest(double a, float f) {
+  const uint64_t u = f64i_bits(a);
+  const int32_t d = int32_t(uint32_t(u) - uint32_t(f64i_bits(f64i_from_f32(f))));
+  // the unit, 2^(e - 1075), as binary32 with a's sign; below its range no rest
+  const int32_t e = int32_t(uint32_t(u >> 52) & 0x7ffu) - 948;
+  const uint32_t unit = (uint32_t(u >> 32) & 0x80000000u) | (uint32_t(e) << 23);
+  return e > 0 && e < 255 ? float(d) * f64i_float(unit) : 0.f;
 }
 
 // float(a): binary64 -> binary32, round to nearest even.
@@ -181,6 +193,27 @@ GBDX_HD double f64i_add(double a, double b) {
   if (r > 0x100u || (r == 0x100u && (q & 1u))) q++;
   if (e + int(q >> 53) > 0x7fe) return f64i_hw_add(a, b);  // overflow
   return f64i_double((ua & 0x8000000000000000ull) | ((uint64_t(e - 1) << 52) + q));
+}
+
+// float(a / b), the place a of a save inside its step of length b: the operands as two
+// binary32 parts each, and one correction of the quotient of the leading parts, which
+// leaves it within 2^-40 of a / b before the last rounding.  Operands so small or large
+// that a part would leave the normal range take the FP64 division.
+GBDX_HD float f64i_quotient_f32(double a, double b) {
+  const float ah = f64i_to_f32(a), bh = f64i_to_f32(b);
+  const float ma = fabsf(ah), mb = fabsf(bh);
+  if (!((ma > 1e-20f || a == 0.0) && ma < 1e18f && mb > 1e-18f && mb < 1e18f))
+    return float(a / b);
+  const float al = f64i_rest(a, ah), bl = f64i_rest(b, bh);
+  float r;
+#ifdef __CUDA_ARCH__
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(bh));
+#else
+  r = 1.f / bh;
+#endif
+  r = fmaf(fmaf(-bh, r, 1.f), r, r);
+  const float q = ah * r;
+  return fmaf(fmaf(-q, bh, ah) + fmaf(-q, bl, al), r, q);
 }
 
 }  // namespace gbdx
