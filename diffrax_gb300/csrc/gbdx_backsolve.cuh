@@ -38,6 +38,7 @@
 #include <cuda_bf16.h>
 
 #include "gbdx_common.cuh"
+#include "gbdx_f2.cuh"
 #include "gbdx_mlp_bwd.cuh"
 #include "gbdx_mma.cuh"
 #include "gbdx_traj.cuh"
@@ -113,13 +114,15 @@ struct BsAct {
 // Operands of the tensor-core parameter pass of one row and one layer
 // W [NO][NI]: o-side vectors U0 = -h u0, A2 = sum_j b_j du_j,
 // A3 = sum_j e_j du_j and the stage differences du_j = -h (u_j - u_0) (BF16,
-// [o][k = j - 1]); i-side vectors v0, B1 = v0 + sum_j b_j dv_j,
-// B3 = sum_j e_j dv_j and b_j dv_j, e_j dv_j (BF16, [k][i]).
+// [o][k = j - 1]); i-side vectors v0, B1 = v0 + sum_j b_j dv_j (pairs of both side by
+// side), B3 = sum_j e_j dv_j and, BF16 [k][i], b_j dv_j over e_j dv_j.  No method has
+// more than eight stage differences, so the products are m16n8k8.
 template <int NO, int NI>
 struct __align__(16) BsLayerOps {
-  float U0[NO], A2[NO], A3[NO], v0[NI], B1[NI], B3[NI];
-  __nv_bfloat16 Du[NO][24];
-  __nv_bfloat16 Bb[16][NI + 8], Be[16][NI + 8];
+  float VB[NI / 2][4];  // v0, v0', B1, B1'
+  float U0[NO], A2[NO], A3[NO], B3[NI];
+  __nv_bfloat16 Du[NO][8];
+  __nv_bfloat16 Bbe[16][NI + 8];
 };
 // The three layers of one row together, so that the row's weight tiles
 // stream as one sequence.
@@ -622,8 +625,8 @@ struct BsLayer<SH, 2> {
 
 // A row's weight tiles as one sequence of batches of U tiles per warp: the
 // one batch of layer 0, the NB1 batches of layer 1, the one batch of layer 2.
-// A batch's a_theta0 loads are issued one batch ahead (two register buffers),
-// across layer and row boundaries.
+// A tile's a_theta0 load is issued one batch ahead, into the registers of the tile just
+// done, across layer and row boundaries.
 template <class SH>
 struct BsTiles {
   template <int L>
@@ -632,6 +635,8 @@ struct BsTiles {
   }
   static constexpr int T0 = tpw<0>(), T1 = tpw<1>(), T2 = tpw<2>();
   static constexpr int U = T0 < 16 ? T0 : 16, NB1 = T1 / U, NB = NB1 + 2;
+  // tiles of one output block in every layer (a row of layer 0 has the fewest)
+  static constexpr int SB = U < SH::D / 8 ? U : SH::D / 8;
   // L2 prefetch distance, in batches: measured best at 2 for the tracked
   // norm's pass (a_theta0 read, the candidate written to the other buffer)
   // and 3 for the in-place pass of the seminorm
@@ -643,7 +648,9 @@ struct BsTiles {
                     T1 * SH::WARPS == (BsLayer<SH, 1>::NO / 16) * (BsLayer<SH, 1>::NI / 8) &&
                     T2 * SH::WARPS == (BsLayer<SH, 2>::NO / 16) * (BsLayer<SH, 2>::NI / 8),
                 "parameter tiles split over the warps");
-  static_assert(T0 == U && T2 == U && T1 % (2 * U) == 0, "parameter tile batches");
+  static_assert(T0 == U && T2 == U && T1 % U == 0, "parameter tile batches");
+  static_assert(U % SB == 0 && SB % 2 == 0 && (SH::D / 8) % SB == 0 && (SH::H / 8) % SB == 0,
+                "tiles of one output block");
 };
 
 // Batch i (0 <= i < NB) of a row in this warp's run: layer 0, NB1 batches of
@@ -676,127 +683,132 @@ __device__ __forceinline__ void batch_prefetch(const float *a0, const float *a0n
   }
 }
 
-// The a_theta0 values of U tiles of layer L from tile tb of this warp's run
-// (zeros for a row whose a_theta is still zero).
-template <class SH, int L>
-__device__ __forceinline__ void batch_load(float (&x)[BsTiles<SH>::U][4], const float *a0,
-                                           int tb, int warp, int lane) {
-  using TL = BsTiles<SH>;
-  constexpr int TPW = TL::template tpw<L>(), WOFF = BsLayer<SH, L>::WOFF;
-#pragma unroll
-  for (int u = 0; u < TL::U; u++) {
-    const int t = warp * TPW + tb + u;
-    if (a0) {
-      const float4 v = __ldcs(reinterpret_cast<const float4 *>(a0 + WOFF + t * 128 + lane * 4));
-      x[u][0] = v.x;
-      x[u][1] = v.y;
-      x[u][2] = v.z;
-      x[u][3] = v.w;
-    } else {
-      x[u][0] = x[u][1] = x[u][2] = x[u][3] = 0.f;
-    }
-  }
+// The a_theta0 values of a tile (zeros for a row whose a_theta is still zero).
+__device__ __forceinline__ void tile_load(float (&x)[4], const float *p) {
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (p) v = __ldcs(reinterpret_cast<const float4 *>(p));
+  x[0] = v.x;
+  x[1] = v.y;
+  x[2] = v.z;
+  x[3] = v.w;
 }
 
-// U tiles of layer L from tile tb: a1 = a0 + da (fragment layout); returns
-// their share of the scaled squared errors when NORM.
-template <class SH, int S, int L, bool NORM>
-__device__ __forceinline__ float batch_tiles(BsPassOps<SH> &pp,
-                                             const float (&x0)[BsTiles<SH>::U][4], float *a1,
-                                             int tb, int warp, int lane, float rtol, float atol) {
-  using TL = BsTiles<SH>;
+// Where a run of tiles of one output block finds its operands.
+struct BsRun {
+  uint32_t a[2];            // A fragment (stage differences)
+  F2 u0a, u0b, a2a, a2b, a3a, a3b;
+  const float *vb, *b3;     // this lane's columns of the first tile
+  const __nv_bfloat16 *be;  // this lane's ldmatrix row
+};
+
+// The run of layer L that begins with tile tf of the layer.
+template <class SH, int L, bool NORM>
+__device__ __forceinline__ void run_src(BsRun &R, BsPassOps<SH> &pp, int tf, int lane) {
   using LY = BsLayer<SH, L>;
-  constexpr int TPW = TL::template tpw<L>(), NI = LY::NI, NTL = NI / 8, WOFF = LY::WOFF;
+  constexpr int NI = LY::NI, NTL = NI / 8;
   auto &ps = LY::ops(pp);
   const int g = lane >> 2, c = lane & 3;
-  float accn = 0.f;
-  // A batch starts on a multiple of U tiles; when U divides the tiles of an
-  // output block, its tiles share one block: its A fragment and o-side
-  // values are loaded once for the batch.
-  constexpr bool ONE_BLOCK = NTL % TL::U == 0;
-  const int tf = warp * TPW + tb;
-  uint32_t ab[4];
-  float u0a_b = 0.f, u0b_b = 0.f, a2a_b = 0.f, a2b_b = 0.f, a3a_b = 0.f, a3b_b = 0.f;
-  if constexpr (ONE_BLOCK) {
-    const int ot = tf / NTL, og = ot * 16 + g;
-    ldsm_a(ab, &ps.Du[ot * 16][0], 24, lane);
-    u0a_b = ps.U0[og];
-    u0b_b = ps.U0[og + 8];
-    a2a_b = ps.A2[og];
-    a2b_b = ps.A2[og + 8];
-    if constexpr (NORM) {
-      a3a_b = ps.A3[og];
-      a3b_b = ps.A3[og + 8];
-    }
+  const int ot = tf / NTL, nt = tf % NTL, og = ot * 16 + g;
+  asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];\n"
+               : "=r"(R.a[0]), "=r"(R.a[1])
+               : "r"(smem_u32(&ps.Du[ot * 16 + (lane & 15)][0])));
+  R.u0a = f2_set(ps.U0[og]);
+  R.u0b = f2_set(ps.U0[og + 8]);
+  R.a2a = f2_set(ps.A2[og]);
+  R.a2b = f2_set(ps.A2[og + 8]);
+  if constexpr (NORM) {
+    R.a3a = f2_set(ps.A3[og]);
+    R.a3b = f2_set(ps.A3[og + 8]);
   }
-#pragma unroll
-  for (int u = 0; u < TL::U; u++) {
-    const int t = tf + u, ot = t / NTL, nt = t % NTL;
-    const int og = ot * 16 + g, ic = nt * 8 + 2 * c;
-    uint32_t a[4], bb[2], be[2];
-    if constexpr (ONE_BLOCK) {
-#pragma unroll
-      for (int k = 0; k < 4; k++) a[k] = ab[k];
-    } else {
-      ldsm_a(a, &ps.Du[ot * 16][0], 24, lane);
-    }
-    ldsm_bt1(bb, &ps.Bb[0][0], NI + 8, 0, nt * 8, lane);
-    const float u0a = ONE_BLOCK ? u0a_b : ps.U0[og], u0b = ONE_BLOCK ? u0b_b : ps.U0[og + 8];
-    const float a2a = ONE_BLOCK ? a2a_b : ps.A2[og], a2b = ONE_BLOCK ? a2b_b : ps.A2[og + 8];
-    const float2 v0 = *reinterpret_cast<const float2 *>(&ps.v0[ic]);
-    const float2 b1 = *reinterpret_cast<const float2 *>(&ps.B1[ic]);
-    float cb[4] = {fmaf(u0a, b1.x, a2a * v0.x), fmaf(u0a, b1.y, a2a * v0.y),
-                   fmaf(u0b, b1.x, a2b * v0.x), fmaf(u0b, b1.y, a2b * v0.y)};
-    if constexpr (S > 1) mma_bf16(cb, a, bb[0], bb[1]);
-    float x1[4];
-#pragma unroll
-    for (int q = 0; q < 4; q++) x1[q] = x0[u][q] + cb[q];
-    if constexpr (NORM) {
-      ldsm_bt1(be, &ps.Be[0][0], NI + 8, 0, nt * 8, lane);
-      const float a3a = ONE_BLOCK ? a3a_b : ps.A3[og], a3b = ONE_BLOCK ? a3b_b : ps.A3[og + 8];
-      const float2 b3 = *reinterpret_cast<const float2 *>(&ps.B3[ic]);
-      float ce[4] = {fmaf(u0a, b3.x, a3a * v0.x), fmaf(u0a, b3.y, a3a * v0.y),
-                     fmaf(u0b, b3.x, a3b * v0.x), fmaf(u0b, b3.y, a3b * v0.y)};
-      if constexpr (S > 1) mma_bf16(ce, a, be[0], be[1]);
-#pragma unroll
-      for (int q = 0; q < 4; q++) accn += scaled_sq(x0[u][q], x1[q], ce[q], rtol, atol);
-    }
-    __stcs(reinterpret_cast<float4 *>(a1 + WOFF + t * 128 + lane * 4),
-           make_float4(x1[0], x1[1], x1[2], x1[3]));
-  }
-  return accn;
+  R.vb = ps.VB[nt * 4 + c];
+  R.b3 = &ps.B3[nt * 8 + 2 * c];
+  // lanes 0-15: b, then e, of a tile's columns; 16-31: of the next tile's
+  R.be = &ps.Bbe[lane & 15][nt * 8 + (lane >> 4) * 8];
 }
 
-// A row's tiles, its layer-0 batch already loading into xa and its first
-// layer-1 batch into xb; ends with batch 0 of the next row (a0n, when next)
-// loading into xa.
+__device__ __forceinline__ void mma_k8(float (&d)[4], const uint32_t (&a)[2], uint32_t b) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k8.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, "
+      "{%0,%1,%2,%3};\n"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(b));
+}
+
+// Tile u of a run: x1 = x0 + da to a1; adds the scaled squared errors when NORM.
+template <int S, bool NORM>
+__device__ __forceinline__ void run_tile(const BsRun &R, int u, const float (&x0)[4],
+                                         uint32_t bb, uint32_t be, float *a1, float rtol,
+                                         float atol, float &accn) {
+  const float4 vb = *reinterpret_cast<const float4 *>(R.vb + 16 * u);
+  const F2 v0 = f2_pack(vb.x, vb.y), b1 = f2_pack(vb.z, vb.w);
+  float cb[4];
+  f2_unpack(f2_fma(R.u0a, b1, f2_mul(R.a2a, v0)), cb[0], cb[1]);
+  f2_unpack(f2_fma(R.u0b, b1, f2_mul(R.a2b, v0)), cb[2], cb[3]);
+  if constexpr (S > 1) mma_k8(cb, R.a, bb);
+  float x1[4];
+  f2_unpack(f2_add(f2_pack(x0[0], x0[1]), f2_pack(cb[0], cb[1])), x1[0], x1[1]);
+  f2_unpack(f2_add(f2_pack(x0[2], x0[3]), f2_pack(cb[2], cb[3])), x1[2], x1[3]);
+  if constexpr (NORM) {
+    const float2 b3f = *reinterpret_cast<const float2 *>(R.b3 + 8 * u);
+    const F2 b3 = f2_pack(b3f.x, b3f.y);
+    float ce[4];
+    f2_unpack(f2_fma(R.u0a, b3, f2_mul(R.a3a, v0)), ce[0], ce[1]);
+    f2_unpack(f2_fma(R.u0b, b3, f2_mul(R.a3b, v0)), ce[2], ce[3]);
+    if constexpr (S > 1) mma_k8(ce, R.a, be);
+#pragma unroll
+    for (int q = 0; q < 4; q++) accn += scaled_sq(x0[q], x1[q], ce[q], rtol, atol);
+  }
+  __stcs(reinterpret_cast<float4 *>(a1 + 128 * u), make_float4(x1[0], x1[1], x1[2], x1[3]));
+}
+
+// A row's tiles, batch by batch; x holds the a_theta0 of its first batch, and each
+// tile's place is loaded again, for the next batch (at the end the next row's first,
+// a0n, when next), as soon as the tile is done.
+// One copy of the 16 tiles' code serves every batch: four unrolled copies, ~70 KB with
+// K = 16 products (half of it zeros) and single FP32 operations, waited on instruction
+// fetches.  4864 trajectories 64-256-256-64 with 32 saves: the backward 67.5 to 57.9 ms
+// (seminorm 61.4 to 57.5), 16384 with their forward 235 to 201 ms; the pass moves a
+// row's 791 KB in 37,000 cycles on all 152 SMs, 6.3 TB/s.
 template <class SH, int S, bool NORM>
-__device__ __forceinline__ float row_tiles(BsPassOps<SH> &pp, float (&xa)[BsTiles<SH>::U][4],
-                                           float (&xb)[BsTiles<SH>::U][4], const float *a0,
-                                           float *a1, bool next, const float *a0n, int warp,
-                                           int lane, float rtol, float atol) {
+__device__ __forceinline__ float row_tiles(BsPassOps<SH> &pp, float (&x)[BsTiles<SH>::U][4],
+                                           const float *a0, float *a1, bool next,
+                                           const float *a0n, int warp, int lane, float rtol,
+                                           float atol) {
   using TL = BsTiles<SH>;
-  constexpr int U = TL::U;
-  float s = batch_tiles<SH, S, 0, NORM>(pp, xa, a1, 0, warp, lane, rtol, atol);
+  constexpr int U = TL::U, SB = TL::SB;
+  float accn = 0.f;
 #pragma unroll 1
-  for (int tb = 0, i = 2; tb < TL::T1; tb += 2 * U, i += 2) {
-    // batch i: layer-1 tile tb + U; batch i + 1: the next
-    batch_load<SH, 1>(xa, a0, tb + U, warp, lane);
-    batch_prefetch<SH>(a0, a0n, next, i + TL::template pf<NORM>(), warp, lane);
-    s += batch_tiles<SH, S, 1, NORM>(pp, xb, a1, tb, warp, lane, rtol, atol);
-    if (tb + 2 * U < TL::T1)
-      batch_load<SH, 1>(xb, a0, tb + 2 * U, warp, lane);
-    else
-      batch_load<SH, 2>(xb, a0, 0, warp, lane);
+  for (int i = 0; i < TL::NB; i++) {
+    const bool wrap = i + 1 == TL::NB;
+    const float *from = wrap ? (next ? a0n : nullptr) : a0;
+    const float *ld = from ? batch_ptr<SH>(from, wrap ? 0 : i + 1, warp) + 4 * lane : nullptr;
+    float *st = const_cast<float *>(batch_ptr<SH>(a1, i, warp)) + 4 * lane;
     batch_prefetch<SH>(a0, a0n, next, i + 1 + TL::template pf<NORM>(), warp, lane);
-    s += batch_tiles<SH, S, 1, NORM>(pp, xa, a1, tb + U, warp, lane, rtol, atol);
+#pragma unroll
+    for (int h = 0; h < U; h += SB) {
+      BsRun R;
+      if (i == 0)
+        run_src<SH, 0, NORM>(R, pp, warp * TL::T0 + h, lane);
+      else if (i <= TL::NB1)
+        run_src<SH, 1, NORM>(R, pp, warp * TL::T1 + (i - 1) * U + h, lane);
+      else
+        run_src<SH, 2, NORM>(R, pp, warp * TL::T2 + h, lane);
+#pragma unroll
+      for (int u = 0; u < SB; u += 2) {
+        uint32_t b[4];
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                     : "=r"(b[0]), "=r"(b[1]), "=r"(b[2]), "=r"(b[3])
+                     : "r"(smem_u32(R.be + 8 * u)));
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+          run_tile<S, NORM>(R, u + q, x[h + u + q], b[2 * q], b[2 * q + 1], st + 128 * h,
+                                  rtol, atol, accn);
+          tile_load(x[h + u + q], ld ? ld + 128 * (h + u + q) : nullptr);
+        }
+      }
+    }
   }
-  if (next) {
-    batch_load<SH, 0>(xa, a0n, 0, warp, lane);
-    batch_prefetch<SH>(a0, a0n, next, TL::NB + TL::template pf<NORM>(), warp, lane);
-  }
-  s += batch_tiles<SH, S, 2, NORM>(pp, xb, a1, 0, warp, lane, rtol, atol);
-  return s;
+  return accn;
 }
 
 // One layer's stage records of a row, loaded into registers (this thread's
@@ -832,14 +844,14 @@ __device__ __forceinline__ float layer_ops(BsPassOps<SH> &pp, const LayerRecs<Ta
   using TB = Tab<SOLVER>;
   using LY = BsLayer<SH, L>;
   constexpr int S = TB::S;
-  static_assert(S - 1 <= 16, "stage differences fit one k16 slice");
+  static_assert(S - 1 <= 8, "stage differences fit one k8 slice");
   auto &ps = LY::ops(pp);
   float accn = 0.f;
   if (tid < LY::NI) {
     const int i = tid;
     float b1 = lr.vv[0], b3 = 0.f;
 #pragma unroll
-    for (int k = 0; k < 16; k++) {
+    for (int k = 0; k < 8; k++) {
       float bb = 0.f, be = 0.f;
       if (k + 1 < S) {
         const float dv = lr.vv[k + 1] - lr.vv[0];
@@ -848,18 +860,18 @@ __device__ __forceinline__ float layer_ops(BsPassOps<SH> &pp, const LayerRecs<Ta
         b1 += bb;
         b3 += be;
       }
-      ps.Bb[k][i] = __float2bfloat16_rn(bb);
-      ps.Be[k][i] = __float2bfloat16_rn(be);
+      ps.Bbe[k][i] = __float2bfloat16_rn(bb);
+      ps.Bbe[8 + k][i] = __float2bfloat16_rn(be);
     }
-    ps.v0[i] = lr.vv[0];
-    ps.B1[i] = b1;
+    ps.VB[i >> 1][i & 1] = lr.vv[0];
+    ps.VB[i >> 1][2 + (i & 1)] = b1;
     ps.B3[i] = b3;
   }
   if (tid < LY::NO) {
     const int o = tid;
     float a2 = 0.f, a3 = 0.f;
 #pragma unroll
-    for (int k = 0; k < 16; k++) {
+    for (int k = 0; k < 8; k++) {
       float du = 0.f;
       if (k + 1 < S) {
         du = lr.uu[k + 1] - lr.uu[0];
@@ -901,8 +913,10 @@ __device__ __forceinline__ void theta_rows_tc(BsPassOps<SH> &pp, float (*rsum)[S
   const float *a0;
   float *a1;
   ptrs(r, a0, a1);
-  float xa[TL::U][4], xb[TL::U][4];
-  batch_load<SH, 0>(xa, a0, 0, warp, lane);
+  float x[TL::U][4];
+#pragma unroll
+  for (int u = 0; u < TL::U; u++)
+    tile_load(x[u], a0 ? batch_ptr<SH>(a0, 0, warp) + 128 * u + 4 * lane : nullptr);
 #pragma unroll
   for (int i = 1; i <= TL::template pf<NORM>(); i++)
     batch_prefetch<SH>(a0, nullptr, false, i, warp, lane);
@@ -917,18 +931,16 @@ __device__ __forceinline__ void theta_rows_tc(BsPassOps<SH> &pp, float (*rsum)[S
     {
       const float xb0 = bias_load<SH, 0>(a0, tid), xb1 = bias_load<SH, 1>(a0, tid),
                   xb2 = bias_load<SH, 2>(a0, tid);
-      batch_load<SH, 1>(xb, a0, 0, warp, lane);
-      batch_prefetch<SH>(a0, a0n, rn < M, 1 + TL::template pf<NORM>(), warp, lane);
-      LayerRecs<S> lr;
-      layer_recs<SH, S, 0>(lr, rec_r, h, xb0, tid);
-      accn = layer_ops<SH, SOLVER, 0, NORM>(pp, lr, a1, rtol, atol, tid);
-      layer_recs<SH, S, 1>(lr, rec_r, h, xb1, tid);
-      accn += layer_ops<SH, SOLVER, 1, NORM>(pp, lr, a1, rtol, atol, tid);
-      layer_recs<SH, S, 2>(lr, rec_r, h, xb2, tid);
-      accn += layer_ops<SH, SOLVER, 2, NORM>(pp, lr, a1, rtol, atol, tid);
+      LayerRecs<S> l0, l1, l2;
+      layer_recs<SH, S, 0>(l0, rec_r, h, xb0, tid);
+      layer_recs<SH, S, 1>(l1, rec_r, h, xb1, tid);
+      layer_recs<SH, S, 2>(l2, rec_r, h, xb2, tid);
+      accn = layer_ops<SH, SOLVER, 0, NORM>(pp, l0, a1, rtol, atol, tid);
+      accn += layer_ops<SH, SOLVER, 1, NORM>(pp, l1, a1, rtol, atol, tid);
+      accn += layer_ops<SH, SOLVER, 2, NORM>(pp, l2, a1, rtol, atol, tid);
     }
     __syncthreads();  // the operands are complete
-    accn += row_tiles<SH, S, NORM>(pp, xa, xb, a0, a1, rn < M, a0n, warp, lane, rtol, atol);
+    accn += row_tiles<SH, S, NORM>(pp, x, a0, a1, rn < M, a0n, warp, lane, rtol, atol);
     if constexpr (NORM) {
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) accn += __shfl_xor_sync(0xffffffffu, accn, o);
