@@ -549,9 +549,6 @@ __global__ void __launch_bounds__((FmShape<D, H>::THREADS), 1) mlp_fm_kernel(Sol
         if (P.save_t0)
           *GBDX_AT(P, reinterpret_cast<float *>(P.ys_out), i * P.n_save * D + m.f, 1,
                    P.batch * P.n_save * D, GBDX_SITE_YS) = Y0[e];
-        if (P.tape_y)
-          *GBDX_AT(P, P.tape_y, i * P.checkpoints * D + m.f, 1, P.batch * P.checkpoints * D,
-                   GBDX_SITE_TAPE_Y) = Y0[e];
         // a resumed row's FSAL value (row_init cleared its `first`)
         if constexpr (XO && TB::FSAL) {
           if (P.state_in && !R.first[row])
@@ -805,7 +802,7 @@ __global__ void __launch_bounds__((FmShape<D, H>::THREADS), 1) mlp_fm_kernel(Sol
       }
       fm_sync(g);
     }
-    // ---- accept: advance the state, FSAL vector, tape -----------------------
+    // ---- accept: advance the state, FSAL vector ----------------------------
     int kept[NE];
     {
       int lv[NE];
@@ -842,21 +839,6 @@ __global__ void __launch_bounds__((FmShape<D, H>::THREADS), 1) mlp_fm_kernel(Sol
         }
         Y0[e] = Y1[e];
         if (TB::FSAL) F0[e] = F[e];  // field value of the last stage (FSAL)
-      }
-    }
-    if (P.tape_y) {
-#pragma unroll
-      for (int e = 0; e < NE; e++) {
-        const int row = m.row0 + e;
-        if (kept[e] && R.cpslot[row] >= 0) {
-          const int64_t b0 = R.idx[row] * P.checkpoints * D + m.f;
-          [[maybe_unused]] const int64_t ext = P.batch * P.checkpoints * D;
-          if (R.cpcompact[row] & 1)
-            for (int s2 = 1; s2 < P.checkpoints / 2; s2++)
-              *GBDX_AT(P, P.tape_y, b0 + s2 * D, 1, ext, GBDX_SITE_TAPE_Y) =
-                  *GBDX_AT(P, P.tape_y, b0 + 2 * s2 * D, 1, ext, GBDX_SITE_TAPE_Y);
-          *GBDX_AT(P, P.tape_y, b0 + R.cpslot[row] * D, 1, ext, GBDX_SITE_TAPE_Y) = Y0[e];
-        }
       }
     }
     // ---- finished rows: t1 save, outputs, refill ----------------------------
@@ -923,10 +905,6 @@ __global__ void __launch_bounds__((FmShape<D, H>::THREADS), 1) mlp_fm_kernel(Sol
         P.stats_out[i * 3 + 0] = R.nsteps[t];
         P.stats_out[i * 3 + 1] = R.nacc[t];
         P.stats_out[i * 3 + 2] = R.nrej[t];
-        if (P.tape_n) {
-          P.tape_n[i] = R.nacc[t];
-          P.tape_stride[i] = R.cpstride[t];
-        }
         R.fin[t] = 1;
         fin = 1;
       }

@@ -71,9 +71,11 @@ OdeEntry mlp_entry(int solver, bool precise, bool sde) {
       return OdeEntry{nullptr, nullptr};
     }
   }
-  // (BF16 ODEs: the feature-major form, gbdx_mlp_fm.cuh)
-  return precise ? mlp_entry_for_solver<D, H, true, false, XO>(solver)
-                 : OdeEntry{nullptr, nullptr};
+  if (precise) return mlp_entry_for_solver<D, H, true, false, XO>(solver);
+  // (BF16 ODEs: only where a gradient tape is recorded, for the shapes with a
+  // recursive backward; the others take the feature-major form, gbdx_mlp_fm.cuh)
+  if constexpr (!XO && H < 256) return mlp_entry_for_solver<D, H, false, false, XO>(solver);
+  return OdeEntry{nullptr, nullptr};
 }
 
 }  // namespace gbdx
