@@ -164,7 +164,7 @@ def lower(terms, solver, stepsize_controller, saveat: SaveAt, *, dim: int, dtype
 
 # The default tape holds every state of an ordinary solve, up to 128, so that the
 # backward recomputes nothing (a training step of 3001 neural ODEs 64-128-128-64 takes
-# 0.90 ms; the segments between ceil(log2(max_steps)) states are recomputed).  Above
+# 0.99 ms; the segments between ceil(log2(max_steps)) states are recomputed).  Above
 # this size it would take a share of the memory that the batch may need: the log2 count.
 _TAPE_BYTES = 16 << 30
 
