@@ -173,9 +173,14 @@ __device__ __forceinline__ void vbt_w(const SolveParams &P, int64_t traj, double
   const float r = float((t - P.vbt_t0) * P.vbt_inv_len);
   const uint32_t tj = uint32_t(traj);
   const int L = P.vbt_levels;
-  uint32_t node;
-  float su, f;  // the leaf interval's length, and r's place in it over its length
-  if (L <= 30) {
+  // The path's node at depth L, the leaf interval's length, and r's place in it over
+  // its length.  A path of more than 30 levels does not fit the word: there node is the
+  // node reached so far (modulo 2^32, as the draws take it) and f is r scaled to the
+  // level reached, and each level takes one more turn.
+  const bool deep = L > 30;
+  uint32_t node = 1;
+  float su, f;
+  if (!deep) {
     // r lies in (i 2^-L, (i + 1) 2^-L]; scaling by 2^L is exact, and from 2^24 on
     // the scaled r is an integer, the interval's end
     const float x = r * __int_as_float((127 + L) << 23);
@@ -184,17 +189,16 @@ __device__ __forceinline__ void vbt_w(const SolveParams &P, int64_t traj, double
     node = (1u << L) + uint32_t(i);
     f = fmaxf(x < 16777216.f ? x - float(i) : 1.f, 0.f);
   } else {
-    float s = 0.f;
-    su = 1.f;
-    node = 1;
-    for (int l = 0; l < L; l++) {
-      su *= 0.5f;
-      const bool right = r > s + su;
-      if (right) s += su;
-      node = 2 * node + (right ? 1u : 0u);
-    }
-    f = fmaxf(r - s, 0.f) / su;
+    su = L < 127 ? __int_as_float((127 - L) << 23) : 0.f;
+    f = fminf(fmaxf(r, 0.f), 1.f);
   }
+  // the child that holds r (deep); the scaled r's last whole place below it is the
+  // child's index, odd once r is the interval's end
+  auto child = [&](uint32_t n) {
+    f += f;
+    const bool right = f >= 16777216.f || (max(int(ceilf(f)) - 1, 0) & 1);
+    return 2 * n + (right ? 1u : 0u);
+  };
   float ws[NQ], wsu[NQ];
   int d = 0;
   const bool cached = C && L <= kVbtCacheLevels;
@@ -221,10 +225,9 @@ __device__ __forceinline__ void vbt_w(const SolveParams &P, int64_t traj, double
     }
   }
   // one level: the halves of the interval of level l, and the one with r
-  auto descend = [&](int l, const float (&z)[NQ]) {
+  auto descend = [&](int l, bool right, const float (&z)[NQ]) {
     // sqrt(2^-l) / 2
     const float a = __int_as_float((126 - ((l + 1) >> 1)) << 23) * (l & 1 ? 1.41421354f : 1.f);
-    const bool right = (node >> (L - l - 1)) & 1u;
 #pragma unroll
     for (int q = 0; q < NQ; q++) {
       const float m = 0.5f * wsu[q];
@@ -245,11 +248,23 @@ __device__ __forceinline__ void vbt_w(const SolveParams &P, int64_t traj, double
 #pragma unroll 1
   for (; l < L; l += 2) {
     const bool leaf = l + 1 == L;
-    vbt_normals2<NQ>(P.seed, tj, node >> (L - l), kVbtMid, node >> (L - l - 1),
-                     leaf ? kVbtLeaf : kVbtMid, quad, sel, z0, z1);
-    descend(l, z0);
-    if (!leaf) descend(l + 1, z1);
+    // the path's nodes at levels l, l + 1 and (unless the leaf is l + 1) l + 2
+    uint32_t n0, n1, n2;
+    if (!deep) {
+      n0 = node >> (L - l);
+      n1 = node >> (L - l - 1);
+      n2 = leaf ? n1 : node >> (L - l - 2);
+    } else {
+      n0 = node;
+      n1 = child(n0);
+      n2 = leaf ? n1 : child(n1);
+      node = n2;
+    }
+    vbt_normals2<NQ>(P.seed, tj, n0, kVbtMid, n1, leaf ? kVbtLeaf : kVbtMid, quad, sel, z0, z1);
+    descend(l, n1 & 1u, z0);
+    if (!leaf) descend(l + 1, n2 & 1u, z1);
   }
+  if (deep) f = f < 16777216.f ? f - fmaxf(ceilf(f) - 1.f, 0.f) : 1.f;
   if (l == L) vbt_normals2<NQ>(P.seed, tj, node, kVbtLeaf, node, kVbtLeaf, quad, sel, z1, z0);
   if (cached) C->node = node;
   float bb;
