@@ -13,6 +13,7 @@ import math
 import threading
 from typing import Any, Optional
 
+import numpy as np
 import torch
 
 from . import _lib
@@ -282,6 +283,19 @@ def _host_checks(t0, t1, dt0, ts, tstride):
             raise RuntimeError("saveat.ts must lie between t0 and t1.")
 
 
+def _check_times(t0, t1, ts):
+    """The saveat.ts checks (_integrate.py:1222-1235) of FP64 numpy arrays, as
+    gbdx_solve_status makes them."""
+    up = t0 < t1  # else time runs backwards
+    down = ~up
+    if ((up.any() and bool((ts[1:] < ts[:-1]).any())) or
+            (down.any() and bool((ts[1:] > ts[:-1]).any()))):
+        raise RuntimeError("saveat.ts must be increasing or decreasing.")
+    lo, hi = np.fmin.reduce(ts), np.fmax.reduce(ts)
+    if bool((up & ((hi > t1) | (lo < t0))).any()) or bool((down & ((lo < t1) | (hi > t0))).any()):
+        raise RuntimeError("saveat.ts must lie between t0 and t1.")
+
+
 class _Status(threading.local):
     """Where gbdx_solve_status leaves a solve's outcome for this thread: per device
     32 device bytes of scratch and 16 of page-locked host memory that the kernel
@@ -291,7 +305,8 @@ class _Status(threading.local):
         self.buffers = {}
 
     def read(self, dev, result, low=None, ts=None):
-        """(unsorted, outside, failed, code), include/gbdx.h; waits for the stream."""
+        """(unsorted, outside, failed, code), include/gbdx.h; waits for the stream.
+        result None: of the times alone."""
         if dev.index != torch.cuda.current_device():
             with torch.cuda.device(dev):
                 return self.read(dev, result, low, ts)
@@ -308,7 +323,8 @@ class _Status(threading.local):
         out = None if addr is not None else torch.empty(4, dtype=torch.int32, device=dev)
         n_ts = 0 if ts is None else ts.numel()
         rc = lib.gbdx_solve_status(
-            result.data_ptr(), result.numel(),
+            None if result is None else result.data_ptr(),
+            low.B if result is None else result.numel(),
             low.t0.data_ptr() if n_ts else None, low.t1.data_ptr() if n_ts else None,
             low.tstride if n_ts else 0, ts.data_ptr() if n_ts else None, n_ts,
             scratch.data_ptr(), addr if out is None else out.data_ptr(), stream.cuda_stream)
@@ -322,13 +338,18 @@ class _Status(threading.local):
 _STATUS = _Status()
 
 
+# Steps up to which a solve is taken to be short enough to find out after it that a save
+# time was invalid.
+_DEFER_STEPS = 1 << 16
+
+
 class Lowered:
     """A lowered, validated solve ready for the C ABI (reused by autograd)."""
 
     def __init__(self, terms, solver, t0, t1, dt0, y0, args, saveat, stepsize_controller,
                  adjoint, max_steps, kernel, block_threads, ctas_per_sm, schedule="auto",
                  want_grad=False, event=None, throw=True, defer_checks=False):
-        dev = _device()
+        dev = self.device = _device()
         # diffrax/_adjoint.py:623-634: the backward solve of BacksolveAdjoint
         # takes the forward's `throw` unless its kwargs override it
         self.throw = bool(throw)
@@ -344,8 +365,12 @@ class Lowered:
         max_steps = _max_steps(max_steps, saveat, want_grad and not isinstance(
             adjoint, BacksolveAdjoint))
         ts = saveat.ts
+        host_ts = None
         if ts is not None:
-            ts = torch.as_tensor(ts, dtype=torch.float64).to(dev).reshape(-1).contiguous()
+            ts = torch.as_tensor(ts, dtype=torch.float64)
+            if ts.device.type == "cpu":
+                host_ts = ts.detach().numpy().reshape(-1)
+            ts = ts.to(dev).reshape(-1).contiguous()
         n_ts = 0 if ts is None else int(ts.numel())
         # the solve's times: SaveAt ts, then a ClipStepSizeController's sorted
         # step_ts and jump_ts (include/gbdx.h)
@@ -372,16 +397,29 @@ class Lowered:
         self.drift = drift
         self.problem = _lib.get_problem(self.fields)
         self.t0, self.t1, self.dt0, self.tstride = _time_arrays(t0, t1, dt0, self.B, dev)
-        # With defer_checks the times in ts are checked with the solve's results
-        # (check()): an invalid time is never or wrongly saved, nothing worse.
-        self.ts_unchecked = ts if defer_checks and n_ts and not _capturing() else None
-        if any(isinstance(x, torch.Tensor) for x in (t0, t1, dt0)):
-            _host_checks(self.t0, self.t1, self.dt0, None if defer_checks else ts, self.tstride)
-        else:
-            if dt0 is not None and (t1 - t0) * dt0 < 0 and not _capturing():
-                raise ValueError("Must have (t1 - t0) * dt0 >= 0")
-            if not defer_checks:
-                _host_checks(self.t0, self.t1, None, ts, self.tstride)
+        # With defer_checks, times that only the device holds are checked with the solve's
+        # results (check()): an invalid time is never or wrongly saved, nothing worse.
+        # Times on the host are checked now, and so are those of a solve that may run long
+        # or that allocates dense records, for one more wait.
+        tensors = any(isinstance(x, torch.Tensor) for x in (t0, t1, dt0))
+        self.ts_unchecked = None
+        if not defer_checks:
+            _host_checks(self.t0, self.t1, self.dt0 if tensors else None, ts, self.tstride)
+        elif tensors:
+            _host_checks(self.t0, self.t1, self.dt0, None, self.tstride)
+        if not tensors and dt0 is not None and not _capturing() and (
+                t1 - t0) * dt0 < 0:
+            raise ValueError("Must have (t1 - t0) * dt0 >= 0")
+        if defer_checks and n_ts and not _capturing():
+            if host_ts is not None and not any(isinstance(x, torch.Tensor) and x.is_cuda
+                                               for x in (t0, t1)):
+                _check_times(*(x.detach().double().numpy().reshape(-1)
+                               if isinstance(x, torch.Tensor) else np.array([float(x)])
+                               for x in (t0, t1)), host_ts)
+            else:
+                self.ts_unchecked = ts
+                if saveat.dense or max_steps > _DEFER_STEPS:
+                    self.check(None, False)
         self.bwd_problem = None
         if backsolve:
             # The backward solve reuses the forward's solver and controller
@@ -433,7 +471,6 @@ class Lowered:
             raise ValueError(f"expected {self.problem.param_count()} field parameters, "
                              f"got {self.params.numel()}")
         self.n_save = self.problem.n_save
-        self.device = dev
 
     def check(self, result, throw):
         """Raises for what was left to check of the times in ts, then (throw) for a
