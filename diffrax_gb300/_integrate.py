@@ -408,7 +408,7 @@ class Lowered:
         elif tensors:
             _host_checks(self.t0, self.t1, self.dt0, None, self.tstride)
         if not tensors and dt0 is not None and not _capturing() and (
-                t1 - t0) * dt0 < 0:
+                float(t1) - float(t0)) * float(dt0) < 0:
             raise ValueError("Must have (t1 - t0) * dt0 >= 0")
         if defer_checks and n_ts and not _capturing():
             if host_ts is not None and not any(isinstance(x, torch.Tensor) and x.is_cuda

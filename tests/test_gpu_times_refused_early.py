@@ -1,5 +1,8 @@
 """Invalid save times are refused before the solve is launched where the host holds every
-time, where the solve has no step bound, and where it would allocate dense records."""
+time, where the solve has no step bound, and where it would allocate dense records; and
+the sign of dt0 is checked for any number that a time may be."""
+from decimal import Decimal
+
 import numpy as np
 import pytest
 import torch
@@ -50,3 +53,10 @@ def test_equal_times():
     with pytest.raises(RuntimeError, match=OUT):
         solve([2.0 + 1e-9], t0=2.0, t1=2.0)
 
+
+@pytest.mark.parametrize("number", [float, Decimal, np.float64, np.float32])
+def test_sign_of_dt0(number):
+    solve([0.5], dt0=number("0.125") if number is Decimal else number(0.125),
+          t0=number(0), t1=number(1))
+    with pytest.raises(ValueError, match="dt0"):
+        solve([0.5], dt0=-0.125, t0=number(0), t1=number(1))
