@@ -49,7 +49,12 @@
 
 namespace gbdx {
 
-constexpr uint32_t kFmWait = 1u << 22;  // polls of a completion barrier
+// Polls of a product's completion barrier before it counts as lost (a test's build sets
+// another number), and of the one that says at the end that none is left in flight.
+#ifndef GBDX_FM_POLLS
+#define GBDX_FM_POLLS (1u << 22)
+#endif
+constexpr uint32_t kFmWait = GBDX_FM_POLLS, kFmDrain = 1u << 22;
 
 template <int D_, int H_>
 struct FmShape {
@@ -92,8 +97,8 @@ struct __align__(128) FmGroup {
   alignas(16) RowState<SH::R> rows;
   float part[SH::R][2];  // the error norm's partial sums
   FmEvents<SH::R, XO> ev;
-  uint64_t bar;
-  int err;
+  uint64_t bar, drain;
+  int err;  // a product of this group did not complete
 };
 
 template <class SH, bool XO>
@@ -252,7 +257,7 @@ struct FmMap {
 
 // F = W2 tanh(W1 tanh(W0 x + b0) + b1) + b2 of the owned elements, for the stage
 // input already written by put() (not yet synchronised).  On return every product
-// has completed; ok is false after a timeout.
+// has completed, or the group's err is set (for all after their next barrier).
 template <class SH, bool XO>
 struct FmEval {
   FmSmem<SH, XO> &sm;
@@ -294,7 +299,10 @@ struct FmEval {
     fm_sync(g);
   }
   __device__ __forceinline__ void wait() {
-    ok = ok && tc::mbar_wait(&gs.bar, phase, kFmWait);
+    if (ok && !tc::mbar_wait(&gs.bar, phase, kFmWait)) {
+      ok = false;
+      *reinterpret_cast<volatile int *>(&gs.err) = 1;
+    }
     phase ^= 1u;
     tc::fence_after_sync();
   }
@@ -320,7 +328,7 @@ struct FmEval {
   }
   __device__ __forceinline__ void operator()(float (&F)[SH::NE]) {
     constexpr int D = SH::D, H = SH::H, N = SH::N;
-    const bool issuer = m.t == 0;
+    const bool issuer = m.t == 0 && ok;
     if constexpr (SH::WIDE) {
 #pragma unroll
       for (int b = 0; b < 2; b++) {
@@ -497,6 +505,7 @@ __global__ void __launch_bounds__((FmShape<D, H>::THREADS), 1) mlp_fm_kernel(Sol
   }
   if (t == 0) {
     tc::mbar_init(&gs.bar, 1);
+    tc::mbar_init(&gs.drain, 1);
     gs.err = 0;
   }
   tc::fence_async_smem();
@@ -626,7 +635,6 @@ __global__ void __launch_bounds__((FmShape<D, H>::THREADS), 1) mlp_fm_kernel(Sol
           for (int e = 0; e < NE; e++) K[j][e] = F[e] * h[e];
         }
     }
-    if (!eval.ok) gs.err = 1;
     // y1, error estimate, per-row scaled error norm
     float Y1[NE];
 #pragma unroll
@@ -842,6 +850,9 @@ __global__ void __launch_bounds__((FmShape<D, H>::THREADS), 1) mlp_fm_kernel(Sol
       }
     }
     // ---- finished rows: t1 save, outputs, refill ----------------------------
+    // (a product that did not complete makes this the group's last step, and every
+    // row that it had a part in an internal error)
+    const bool lost = *reinterpret_cast<volatile int *>(&gs.err);
     int fin = 0;
     if (t < M) {
       R.fin[t] = 0;
@@ -901,6 +912,7 @@ __global__ void __launch_bounds__((FmShape<D, H>::THREADS), 1) mlp_fm_kernel(Sol
         int res = R.result[t];
         if (res == GBDX_SUCCESSFUL && order_key(R.tprev[t]) < order_key(R.t1[t]))
           res = GBDX_MAX_STEPS_REACHED;
+        if (lost) res = GBDX_INTERNAL_ERROR;
         P.result_out[i] = res;
         P.stats_out[i * 3 + 0] = R.nsteps[t];
         P.stats_out[i * 3 + 1] = R.nacc[t];
@@ -935,15 +947,30 @@ __global__ void __launch_bounds__((FmShape<D, H>::THREADS), 1) mlp_fm_kernel(Sol
         }
       }
       fm_sync(g);
-      if (t < M && R.fin[t]) take(queued + atomicAdd(P.queue, 1ull));
+      if (t < M && R.fin[t]) {
+        if (lost)
+          R.active[t] = 0;
+        else
+          take(queued + atomicAdd(P.queue, 1ull));
+      }
       fm_sync(g);
       load();
       fm_sync(g);
       if (t < M) R.loaded[t] = 0;
     }
-    // a product that did not complete ends the group's rows with an internal error
-    if (gs.err) {
-      if (t < M && R.active[t]) P.result_out[R.idx[t]] = GBDX_INTERNAL_ERROR;
+    if (lost) {
+      // the rows still under way, and those that no group may be left to take
+      if (t < M) {
+        if (R.active[t]) P.result_out[R.idx[t]] = GBDX_INTERNAL_ERROR;
+        for (unsigned long long q = queued + atomicAdd(P.queue, 1ull);
+             q < (unsigned long long)P.batch; q = queued + atomicAdd(P.queue, 1ull))
+          P.result_out[P.order ? (int64_t)P.order[q] : (int64_t)q] = GBDX_INTERNAL_ERROR;
+      }
+      // the operands and accumulators stay until no product uses them
+      if (t == 0) {
+        tc::mma_commit(&gs.drain);
+        tc::mbar_wait(&gs.drain, 0, kFmDrain);
+      }
       break;
     }
   }
