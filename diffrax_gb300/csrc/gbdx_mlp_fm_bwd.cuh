@@ -167,7 +167,10 @@ __device__ void fb_issuer(FbSmem<SH> &sm, uint32_t tmem) {
   const bool lead = (threadIdx.x & 31) == 0;
   while (true) {
     fb_await(kFbWant);
-    const int job = *reinterpret_cast<volatile int *>(&sm.job);
+    // the leading lane's: its product lets the others post the next job, which a lane
+    // behind it would read
+    const int job =
+        __shfl_sync(0xffffffffu, *reinterpret_cast<volatile int *>(&sm.job), 0);
     if (job == kFbExit) return;
     if (lead) {
       tc::fence_after_sync();
