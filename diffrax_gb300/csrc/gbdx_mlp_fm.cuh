@@ -257,7 +257,7 @@ struct FmMap {
 
 // F = W2 tanh(W1 tanh(W0 x + b0) + b1) + b2 of the owned elements, for the stage
 // input already written by put() (not yet synchronised).  On return every product
-// has completed, or the group's err is set (for all after their next barrier).
+// has completed; ok is false after a timeout.
 template <class SH, bool XO>
 struct FmEval {
   FmSmem<SH, XO> &sm;
@@ -299,10 +299,7 @@ struct FmEval {
     fm_sync(g);
   }
   __device__ __forceinline__ void wait() {
-    if (ok && !tc::mbar_wait(&gs.bar, phase, kFmWait)) {
-      ok = false;
-      *reinterpret_cast<volatile int *>(&gs.err) = 1;
-    }
+    ok = ok && tc::mbar_wait(&gs.bar, phase, kFmWait);
     phase ^= 1u;
     tc::fence_after_sync();
   }
@@ -328,7 +325,7 @@ struct FmEval {
   }
   __device__ __forceinline__ void operator()(float (&F)[SH::NE]) {
     constexpr int D = SH::D, H = SH::H, N = SH::N;
-    const bool issuer = m.t == 0 && ok;
+    const bool issuer = m.t == 0;
     if constexpr (SH::WIDE) {
 #pragma unroll
       for (int b = 0; b < 2; b++) {
@@ -635,6 +632,7 @@ __global__ void __launch_bounds__((FmShape<D, H>::THREADS), 1) mlp_fm_kernel(Sol
           for (int e = 0; e < NE; e++) K[j][e] = F[e] * h[e];
         }
     }
+    if (!eval.ok) gs.err = 1;
     // y1, error estimate, per-row scaled error norm
     float Y1[NE];
 #pragma unroll
@@ -695,6 +693,7 @@ __global__ void __launch_bounds__((FmShape<D, H>::THREADS), 1) mlp_fm_kernel(Sol
           if (ev_steady && fm_sync_or(g, t < M && live && R.keep[t])) {
             eval.put(Y1);
             eval(F);
+            if (!eval.ok) gs.err = 1;
           }
         }
         if (m.f < 4) {
