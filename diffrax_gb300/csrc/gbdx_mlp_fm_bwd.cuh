@@ -67,7 +67,9 @@ struct __align__(128) FbSmem {
   BwdRows<SH::R> rows;
   float bias[4][SH::GT];
   uint64_t bar, barw;  // a chain product is done; a weight-gradient product is
+  uint64_t drain;
   int job;
+  int issued, issuedw;  // products of either kind issued so far
   uint32_t slot;
   int err;
 };
@@ -160,18 +162,27 @@ __device__ __forceinline__ void fb_await(int id) {
 }
 
 // The issuing warp: runs the wanted products until told to leave (the others always
-// tell it, after a timeout of theirs too).
+// tell it, after a timeout of theirs too: FbField::wait).
 template <class SH>
 __device__ void fb_issuer(FbSmem<SH> &sm, uint32_t tmem) {
   constexpr int D = SH::D, H = SH::H, N = SH::N, R = SH::R, MW = SH::MW;
   const bool lead = (threadIdx.x & 31) == 0;
+  int issued = 0, issuedw = 0;
   while (true) {
     fb_await(kFbWant);
     // the leading lane's: its product lets the others post the next job, which a lane
     // behind it would read
     const int job =
         __shfl_sync(0xffffffffu, *reinterpret_cast<volatile int *>(&sm.job), 0);
-    if (job == kFbExit) return;
+    if (job == kFbExit) {
+      // the operands and accumulators stay until no product uses them
+      if (lead && *reinterpret_cast<volatile int *>(&sm.err)) {
+        tc::mma_commit(&sm.drain);
+        tc::mbar_wait(&sm.drain, 0, kFmDrain);
+      }
+      __syncwarp();
+      return;
+    }
     if (lead) {
       tc::fence_after_sync();
       switch (job) {
@@ -189,6 +200,7 @@ __device__ void fb_issuer(FbSmem<SH> &sm, uint32_t tmem) {
           break;
       }
       tc::mma_commit(&sm.bar);
+      *reinterpret_cast<volatile int *>(&sm.issued) = ++issued;
     }
     __syncwarp();
     if (job < kFbB2) continue;
@@ -204,6 +216,7 @@ __device__ void fb_issuer(FbSmem<SH> &sm, uint32_t tmem) {
           break;
       }
       tc::mma_commit(&sm.barw);
+      *reinterpret_cast<volatile int *>(&sm.issuedw) = ++issuedw;
     }
     __syncwarp();
   }
@@ -299,6 +312,17 @@ __device__ __forceinline__ void fb_brownian(const SolveParams &P, const BwdRows<
   }
 }
 
+// A product did not complete: err is set, and the thread goes on (false) once product n
+// has been issued.  So it stays behind the issuing warp, as the barriers between them
+// need, and the walk ends with the iteration.  Out of line: in each of the nine waits it
+// cost the 32-64 neural SDE 4 % (9001 rows: 5.93 -> 6.15 ms).
+static __device__ __noinline__ bool fb_lost(int *err, const int *issued, int n) {
+  *reinterpret_cast<volatile int *>(err) = 1;
+  for (uint32_t i = 0; i < kFmDrain && *reinterpret_cast<const volatile int *>(issued) <= n; i++)
+    __nanosleep(100);
+  return false;
+}
+
 // The products of the field and its VJP, from the threads that own elements.
 template <class SH>
 struct FbField {
@@ -308,7 +332,7 @@ struct FbField {
   const FmMap<SH> &m;
   const uint32_t tmem;
   const float b0, b1, b2, bs;
-  uint32_t phase = 0, phasew = 0;
+  uint32_t done = 0, donew = 0;  // products of either kind waited for
   bool ok = true, pending = false;
   bool first = true;  // no weight gradient of this iteration yet
   FbSum d0, d1, d2, ds;  // bias gradients of the thread's features and rows
@@ -329,17 +353,16 @@ struct FbField {
     tc::fence_before_sync();
     fb_arrive(kFbFree);
   }
-  __device__ __forceinline__ void wait(uint64_t *bar, uint32_t &ph) {
-    if (!ok) {
-      // after a timeout: stay behind the issuing warp until the walk ends
-      __nanosleep(20000);
-    } else if (!tc::mbar_wait(bar, ph, kFmWait)) {
-      ok = false;
-      *reinterpret_cast<volatile int *>(&sm.err) = 1;
-    }
-    ph ^= 1u;
+  // The next product on bar is complete.  Once one was not within the limit (err), the
+  // thread goes on when it has been issued: it stays behind the issuing warp, as the
+  // barriers between them need, and the walk ends with the iteration.
+  __device__ __forceinline__ void wait(uint64_t *bar, uint32_t &n, const int *issued) {
+    if (!ok || !tc::mbar_wait(bar, n & 1u, kFmWait)) ok = fb_lost(&sm.err, issued, int(n));
+    n++;
     tc::fence_after_sync();
   }
+  __device__ __forceinline__ void wait_chain() { wait(&sm.bar, done, &sm.issued); }
+  __device__ __forceinline__ void wait_weights() { wait(&sm.barw, donew, &sm.issuedw); }
   // the weight-gradient product in flight is done: NC columns to the sum at dst
   template <int NC>
   __device__ __forceinline__ void collect(int src, int dst) {
@@ -354,7 +377,7 @@ struct FbField {
   }
   __device__ __forceinline__ void drain() {
     if (!pending) return;
-    wait(&sm.barw, phasew);
+    wait_weights();
     collect_last();
   }
   __device__ __forceinline__ void put(__nv_bfloat16 *buf, const float (&Y)[NE]) {
@@ -389,11 +412,11 @@ struct FbField {
   // x, a1, a2 of the stage input Y; F (unless last_only) and sigma
   __device__ __forceinline__ void forward(const float (&Y)[NE], float (&F)[NE],
                                           float (&sig)[NE], bool want_f) {
-    if (pending) wait(&sm.barw, phasew);  // (the last stage's products read x)
+    if (pending) wait_weights();  // (the last stage's products read x)
     put(sm.x, Y);
     post(kFbF0);
     if (pending) collect_last();
-    wait(&sm.bar, phase);
+    wait_chain();
     if constexpr (SH::SDE) {
       owned(m.lanes + SH::N, bs, sig);
 #pragma unroll
@@ -402,11 +425,11 @@ struct FbField {
     }
     hidden(b0, sm.a1);
     post(kFbF1);
-    wait(&sm.bar, phase);
+    wait_chain();
     hidden(b1, sm.a2);
     if (want_f) {
       post(kFbF2);
-      wait(&sm.bar, phase);
+      wait_chain();
       owned(m.lanes, b2, F);
     }
   }
@@ -452,20 +475,20 @@ struct FbField {
     }
     post(kFbB2);
     release();
-    wait(&sm.bar, phase);
+    wait_chain();
     back(sm.a2, sm.g2, d1);
     // a gradient is collected while the next product of the chain runs
     post(kFbB1);
-    wait(&sm.barw, phasew);
+    wait_weights();
     collect<D>(SH::TA, SH::T2);
     release();
-    wait(&sm.bar, phase);
+    wait_chain();
     back(sm.a1, sm.g1, d0);
     post(kFbB0);
-    wait(&sm.barw, phasew);
+    wait_weights();
     collect<H>(SH::TA, SH::T1);
     release();
-    wait(&sm.bar, phase);
+    wait_chain();
     pending = true;
     owned(m.lanes, 0.f, gY);
   }
@@ -548,7 +571,8 @@ __global__ void __launch_bounds__((FbShape<D, H, SDE>::THREADS), 1)
   if (t == 0) {
     tc::mbar_init(&sm.bar, 1);
     tc::mbar_init(&sm.barw, 1);
-    sm.err = 0;
+    tc::mbar_init(&sm.drain, 1);
+    sm.err = sm.issued = sm.issuedw = 0;
   }
   tc::fence_async_smem();
   tc::fence_before_sync();
@@ -849,6 +873,9 @@ __global__ void __launch_bounds__((FbShape<D, H, SDE>::THREADS), 1)
           }
         }
       }
+      // a product that did not complete makes this the last iteration, and leaves no
+      // gradients of the rows that it had a part in
+      const bool lost = *reinterpret_cast<volatile int *>(&sm.err);
       if (fm_sync_or(0, fin)) {
         // finished rows: dL/dy0 (plus the t0 save's cotangent)
 #pragma unroll
@@ -858,18 +885,29 @@ __global__ void __launch_bounds__((FbShape<D, H, SDE>::THREADS), 1)
             const int64_t i = R.idx[row];
             float g = GY[e];
             if (P.save_t0) g += Q.grad_ys[(i * n_save) * D + m.f];
-            Q.grad_y0[i * D + m.f] = g;
+            Q.grad_y0[i * D + m.f] = lost ? NAN : g;
           }
         }
         fm_sync(0);
-        if (t < M && R.fin[t]) take(queued + atomicAdd(P.queue, 1ull));
+        if (t < M && R.fin[t]) {
+          if (lost)
+            R.active[t] = 0;
+          else
+            take(queued + atomicAdd(P.queue, 1ull));
+        }
       }
       fm_sync(0);
-      // a product that did not complete leaves no gradients
-      if (*reinterpret_cast<volatile int *>(&sm.err)) {
+      if (lost) {
+        // the rows still under way, and those that no CTA may be left to take
 #pragma unroll
         for (int e = 0; e < NE; e++)
           if (R.active[m.row0 + e]) Q.grad_y0[R.idx[m.row0 + e] * D + m.f] = NAN;
+        if (t < M)
+          for (unsigned long long q = queued + atomicAdd(P.queue, 1ull);
+               q < (unsigned long long)P.batch; q = queued + atomicAdd(P.queue, 1ull)) {
+            const int64_t i = P.order ? (int64_t)P.order[q] : (int64_t)q;
+            for (int d = 0; d < D; d++) Q.grad_y0[i * D + d] = NAN;
+          }
         break;
       }
       load_rows();
@@ -883,6 +921,8 @@ __global__ void __launch_bounds__((FbShape<D, H, SDE>::THREADS), 1)
     sm.bias[2][t] = field.d2.s;
     sm.bias[3][t] = field.ds.s;
     fm_sync(0);
+    if (sm.err)
+      for (int p = t; p < Q.n_params; p += SH::GT) psum[p] = NAN;
     auto total = [&](int which, int width) {
       FbSum s;
       for (int k = t; k < SH::GT; k += width) s.add(sm.bias[which][k]);

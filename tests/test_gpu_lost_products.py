@@ -35,7 +35,7 @@ def impatient(tmp_path_factory):
     return lib
 
 
-@pytest.mark.parametrize("way", ["fwd"])
+@pytest.mark.parametrize("way", ["fwd", "bwd"])
 def test_lost_products(impatient, way):
     env = dict(os.environ, PYTHONPATH=os.pathsep.join(
         [os.path.dirname(HERE), os.environ.get("PYTHONPATH", "")]))
