@@ -14,6 +14,7 @@
 
 #include "../../include/gbdx.h"
 #include "gbdx_launch.h"
+#include "gbdx_tape.h"
 #include "gbdx_sched.h"
 
 namespace {
@@ -154,7 +155,7 @@ int ws_layout(const gbdx_problem *p, int64_t batch, WsLayout *L) {
     L->pcomp = off;
     L->n_cta = int(B);
   } else if (d.adjoint == GBDX_ADJ_RECURSIVE && p->bwd.launch) {
-    const int C = d.checkpoints > 1 ? d.checkpoints : 2;
+    const int C = gbdx::tape_slots(d.checkpoints);
     L->tape_t = off;
     off += up256(B * size_t(d.max_steps + 1) * sizeof(double));
     L->tape_y = off;
@@ -163,9 +164,7 @@ int ws_layout(const gbdx_problem *p, int64_t batch, WsLayout *L) {
     off += up256(B * sizeof(int32_t));
     L->tape_s = off;
     off += up256(B * sizeof(int32_t));
-    // With C slots the checkpoint stride stays below 2 max_steps / C + 1.
-    int seg = (2 * d.max_steps + C - 1) / C + 1;
-    if (seg > d.max_steps + 1) seg = d.max_steps + 1;
+    const int seg = gbdx::tape_segment(d.max_steps, C);
     L->seg_max = seg;
     L->scratch = off;
     off += up256(B * size_t(seg) * d.dim * sizeof(float));
@@ -808,12 +807,10 @@ static int prepare(const gbdx_problem *problem, int64_t batch, const double *t0,
     P.tape_y = reinterpret_cast<float *>(w + L->tape_y);
     P.tape_n = reinterpret_cast<int32_t *>(w + L->tape_n);
     P.tape_stride = reinterpret_cast<int32_t *>(w + L->tape_s);
-    // An even slot count keeps the online thinning exact: when the slots
-    // fill at step n = C s, n is a multiple of the doubled stride 2 s.  The
-    // plain form tapes every accepted step.
+    // (the plain form tapes every accepted step)
     P.checkpoints = (d.kernel == GBDX_KERNEL_PLAIN || problem->adj.rc_bwd)
                         ? d.max_steps + 1
-                        : (d.checkpoints >= 4 ? (d.checkpoints / 2) * 2 : 2);
+                        : gbdx::tape_slots(d.checkpoints);
   }
   return GBDX_OK;
 }
