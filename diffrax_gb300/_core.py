@@ -564,9 +564,11 @@ class AbstractAdjoint:
 @dataclasses.dataclass(frozen=True)
 class RecursiveCheckpointAdjoint(AbstractAdjoint):
     """diffrax/_adjoint.py:179-312.  `checkpoints` bounds the per-trajectory
-    checkpoint slots; None means 128 (the reference: ceil(log2(max_steps))): longer
-    checkpoint segments would take more memory in recomputed states than the slots
-    save, and a second pass over the steps."""
+    checkpoint slots.  None (the reference: ceil(log2(max_steps))) means up to 128, and
+    at most max_steps: solves of fewer steps recompute nothing.  A tape that would pass
+    1 GiB has at most as many as take no more memory, with the states recomputed between
+    two of them, than ceil(log2(max_steps)) would; from max_steps of about 640 on that is
+    all 128."""
     checkpoints: Optional[int] = None
 
 

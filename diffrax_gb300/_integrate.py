@@ -165,18 +165,36 @@ def lower(terms, solver, stepsize_controller, saveat: SaveAt, *, dim: int, dtype
 
 # The default tape holds every state of an ordinary solve, up to 128, so that the
 # backward recomputes nothing (a training step of 3001 neural ODEs 64-128-128-64 takes
-# 0.99 ms; the segments between ceil(log2(max_steps)) states are recomputed).  Above
-# this size it would take a share of the memory that the batch may need: the log2 count.
-_TAPE_BYTES = 16 << 30
+# 0.99 ms; the segments between ceil(log2(max_steps)) states are recomputed).  A tape
+# above this size takes no more memory than that count's would.
+_TAPE_BYTES = 1 << 30
 
 
 def _default_checkpoints(max_steps, state_bytes=0):
     """Tape states of a recursive adjoint without a count, for a batch whose states
-    take state_bytes."""
+    take state_bytes, before _tape_count looks at the segments between them."""
     cp = min(128, max(2, int(max_steps) // 2 * 2))
     if cp * state_bytes > _TAPE_BYTES:
         cp = min(cp, max(1, math.ceil(math.log2(max(int(max_steps), 2)))))
     return cp
+
+
+def _tape_states(max_steps, checkpoints):
+    """States a trajectory takes in the workspace: the tape's and the recomputed ones
+    between two of them (csrc/gbdx_tape.h)."""
+    c = checkpoints // 2 * 2 if checkpoints >= 4 else 2
+    return c + min(-(-2 * max_steps // c) + 1, max_steps + 1)
+
+
+def _tape_count(max_steps, state_bytes):
+    """The default count of a batch: where the tape would be large, the most states that
+    take no more memory with their segments than the log2 count with its long ones (all
+    128 from 640 steps on: at the default 4096 193 states, and 696 with 12)."""
+    max_steps = int(max_steps)
+    cp = _default_checkpoints(max_steps, state_bytes)
+    room = _tape_states(max_steps, cp)
+    most = _default_checkpoints(max_steps)
+    return max([c for c in range(2, most + 1, 2) if _tape_states(max_steps, c) <= room])
 
 
 def _cuda() -> bool:
@@ -391,7 +409,7 @@ class Lowered:
                             block_threads=block_threads, ctas_per_sm=ctas_per_sm,
                             schedule=schedule, event=event)
         if self.fields["adjoint"] == 1 and self.adjoint.checkpoints is None:
-            self.fields["checkpoints"] = _default_checkpoints(
+            self.fields["checkpoints"] = _tape_count(
                 max_steps, self.B * self.dim * self.dtype.itemsize)
         drift = _split_terms(terms)[0]
         self.drift = drift
