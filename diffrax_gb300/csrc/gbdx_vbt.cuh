@@ -39,10 +39,13 @@ enum { kVbtRoot = 0, kVbtMid = 1, kVbtLeaf = 2, kVbtRootH = 3, kVbtMidH = 4, kVb
 // ub, vb in z[2], z[3].  A draw costs as much as the rest of the descent, so the
 // functions are spelled out on the packed FP32x2 pipe: log as e ln 2 + log1p(f), u
 // = (1 + f) 2^e with 1 + f in [sqrt 1/2, sqrt 2) and a minimax fit (6e-9 relative);
-// cos and sin of pi/2 r, r the distance of 4 v from its quadrant (fits 3e-9, 5e-11
-// relative; v needs no other reduction).  Each value is within about two units in
-// the last place, as logf, sqrtf and sincospif give it, at a third of their issue
-// slots.
+// cos and sin of pi/2 r, r the distance of 4 v from its quadrant (fits 1e-8, 4e-8
+// relative, most of the latter the FP32 rounding of pi/2; v needs no other reduction).
+// A third of the issue slots of logf, sqrtf and sincospif.  Error against FP64: rms
+// 4.8e-8 (theirs 4.4e-8), at most 6.9e-7 (5.9e-7); sums over a tree's levels round by as
+// much, and solves come out as far from 64 bits as with the library's functions (the
+// Ornstein--Uhlenbeck paths 2.1e-7, the neural SDE's 3.9e-7).  A sine with pi/2 in two
+// parts and a rounded root (rms 4.5e-8) cost those solves 7 and 3 %.
 __device__ __forceinline__ void box_muller2(uint32_t ua, uint32_t va, uint32_t ub, uint32_t vb,
                                             float (&z)[4]) {
   // (k + 1/2) 2^-24 = (2 k + 1) 2^-25, one rounding
