@@ -798,8 +798,10 @@ static int prepare(const gbdx_problem *problem, int64_t batch, const double *t0,
   // GB300 issues FP64 at ~1/64 of the FP32 rate: the per-evaluation division
   // and square root of the tree's time scaling are done once here.
   P.vbt_inv_len = 1.0 / (d.vbt_t1 - d.vbt_t0);
-  P.vbt_levels = 0;
-  for (float su = 1.f; su > float(P.vbt_tol_unit) && P.vbt_levels < 160; su *= 0.5f) P.vbt_levels++;
+  int levels = 0;
+  for (float su = 1.f; su > float(P.vbt_tol_unit) && levels < 160; su *= 0.5f) levels++;
+  P.vbt_deep = levels > gbdx::kVbtWordLevels ? levels : 0;
+  P.vbt_levels = levels > gbdx::kVbtWordLevels ? gbdx::kVbtWordLevels : levels;
   P.vbt_sqrt_len = float(sqrt(d.vbt_t1 - d.vbt_t0));
   if (d.adjoint == GBDX_ADJ_RECURSIVE && (problem->bwd.launch || problem->adj.rc_bwd)) {
     char *w = static_cast<char *>(workspace);

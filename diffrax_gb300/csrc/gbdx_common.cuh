@@ -480,6 +480,9 @@ struct FieldLevy<F, decltype(void(F::LEVY))> {
   static constexpr bool value = F::LEVY;
 };
 
+// Levels of a Brownian tree whose path a 32-bit node number holds.
+constexpr int kVbtWordLevels = 30;
+
 // ---------------------------------------------------------------------------
 // Kernel parameters shared by every analytic-field launch.
 // ---------------------------------------------------------------------------
@@ -514,7 +517,9 @@ struct SolveParams {
   uint64_t seed;              // Brownian generator seed
   double vbt_t0, vbt_len, vbt_tol_unit;
   double vbt_inv_len;         // 1 / vbt_len
-  int vbt_levels;             // least level with 2^-level <= vbt_tol_unit (in FP32)
+  // least level with 2^-level <= vbt_tol_unit (in FP32): vbt_levels up to kVbtWordLevels,
+  // of deeper trees vbt_deep (else 0)
+  int vbt_levels, vbt_deep;
   float vbt_sqrt_len;         // sqrt(vbt_len) as FP32
   // Recursive-checkpoint tape (forward pass of a differentiated solve)
   double *tape_t;             // [batch, max_steps + 1] accepted-step time grid

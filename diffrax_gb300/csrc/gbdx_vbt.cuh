@@ -166,6 +166,7 @@ using VbtQuadCache = VbtCache<4>;
 // holds r (the left one at its midpoint), down to 2^-level <= tol.  The path is known
 // from r alone, so the levels' normals are drawn two at a time (the leaf's with the
 // last) and the short bridge recursion follows.  C (may be null): the cached path.
+// Trees of at most kVbtWordLevels levels, whose path a 32-bit node holds.
 // Bound: issue slots, ~96 a warp and Philox block and ~112 a pair of Box--Muller
 // pairs.  The Ornstein--Uhlenbeck solve of 16384 paths and 100 steps (under one warp
 // a scheduler, so the overlapped draws count most) went from 0.82 to 0.49 ms, the
@@ -176,32 +177,13 @@ __device__ __forceinline__ void vbt_w(const SolveParams &P, int64_t traj, double
   const float r = float((t - P.vbt_t0) * P.vbt_inv_len);
   const uint32_t tj = uint32_t(traj);
   const int L = P.vbt_levels;
-  // The path's node at depth L, the leaf interval's length, and r's place in it over
-  // its length.  A path of more than 30 levels does not fit the word: there node is the
-  // node reached so far (modulo 2^32, as the draws take it) and f is r scaled to the
-  // level reached, and each level takes one more turn.
-  const bool deep = L > 30;
-  uint32_t node = 1;
-  float su, f;
-  if (!deep) {
-    // r lies in (i 2^-L, (i + 1) 2^-L]; scaling by 2^L is exact, and from 2^24 on
-    // the scaled r is an integer, the interval's end
-    const float x = r * __int_as_float((127 + L) << 23);
-    su = __int_as_float((127 - L) << 23);
-    const int i = max(0, min(int(ceilf(x)) - 1, (1 << L) - 1));
-    node = (1u << L) + uint32_t(i);
-    f = fmaxf(x < 16777216.f ? x - float(i) : 1.f, 0.f);
-  } else {
-    su = L < 127 ? __int_as_float((127 - L) << 23) : 0.f;
-    f = fminf(fmaxf(r, 0.f), 1.f);
-  }
-  // the child that holds r (deep); the scaled r's last whole place below it is the
-  // child's index, odd once r is the interval's end
-  auto child = [&](uint32_t n) {
-    f += f;
-    const bool right = f >= 16777216.f || (max(int(ceilf(f)) - 1, 0) & 1);
-    return 2 * n + (right ? 1u : 0u);
-  };
+  // r lies in (i 2^-L, (i + 1) 2^-L]; scaling by 2^L is exact, and from 2^24 on the
+  // scaled r is an integer, the interval's end.  node: the leaf interval's; su: its
+  // length, f: r's place in it over its length.
+  const float x = r * __int_as_float((127 + L) << 23), su = __int_as_float((127 - L) << 23);
+  const int i = max(0, min(int(ceilf(x)) - 1, (1 << L) - 1));
+  const uint32_t node = (1u << L) + uint32_t(i);
+  const float f = fmaxf(x < 16777216.f ? x - float(i) : 1.f, 0.f);
   float ws[NQ], wsu[NQ];
   int d = 0;
   const bool cached = C && L <= kVbtCacheLevels;
@@ -228,9 +210,10 @@ __device__ __forceinline__ void vbt_w(const SolveParams &P, int64_t traj, double
     }
   }
   // one level: the halves of the interval of level l, and the one with r
-  auto descend = [&](int l, bool right, const float (&z)[NQ]) {
+  auto descend = [&](int l, const float (&z)[NQ]) {
     // sqrt(2^-l) / 2
     const float a = __int_as_float((126 - ((l + 1) >> 1)) << 23) * (l & 1 ? 1.41421354f : 1.f);
+    const bool right = (node >> (L - l - 1)) & 1u;
 #pragma unroll
     for (int q = 0; q < NQ; q++) {
       const float m = 0.5f * wsu[q];
@@ -251,23 +234,11 @@ __device__ __forceinline__ void vbt_w(const SolveParams &P, int64_t traj, double
 #pragma unroll 1
   for (; l < L; l += 2) {
     const bool leaf = l + 1 == L;
-    // the path's nodes at levels l, l + 1 and (unless the leaf is l + 1) l + 2
-    uint32_t n0, n1, n2;
-    if (!deep) {
-      n0 = node >> (L - l);
-      n1 = node >> (L - l - 1);
-      n2 = leaf ? n1 : node >> (L - l - 2);
-    } else {
-      n0 = node;
-      n1 = child(n0);
-      n2 = leaf ? n1 : child(n1);
-      node = n2;
-    }
-    vbt_normals2<NQ>(P.seed, tj, n0, kVbtMid, n1, leaf ? kVbtLeaf : kVbtMid, quad, sel, z0, z1);
-    descend(l, n1 & 1u, z0);
-    if (!leaf) descend(l + 1, n2 & 1u, z1);
+    vbt_normals2<NQ>(P.seed, tj, node >> (L - l), kVbtMid, node >> (L - l - 1),
+                     leaf ? kVbtLeaf : kVbtMid, quad, sel, z0, z1);
+    descend(l, z0);
+    if (!leaf) descend(l + 1, z1);
   }
-  if (deep) f = f < 16777216.f ? f - fmaxf(ceilf(f) - 1.f, 0.f) : 1.f;
   if (l == L) vbt_normals2<NQ>(P.seed, tj, node, kVbtLeaf, node, kVbtLeaf, quad, sel, z1, z0);
   if (cached) C->node = node;
   float bb;
@@ -277,20 +248,67 @@ __device__ __forceinline__ void vbt_w(const SolveParams &P, int64_t traj, double
   for (int q = 0; q < NQ; q++) w[q] = sq * (ws[q] + f * wsu[q] + bb * z1[q]);
 }
 
+// The same for dimensions (col, col + 1) of a deeper tree, level by level: each takes the
+// turn that r scaled to it says, and the node's number is kept modulo 2^32, as the draws
+// take it.  (A function of its own, one pair and one level at a time: its registers count
+// for every kernel that may call it, and 80 are what lets three CTAs of the neural SDE
+// share an SM; with turns of both kinds in vbt_w 32768 trajectories took 3.40 instead of
+// 3.33 ms, with a copy of vbt_w for quads 3.9.)
+static __device__ __noinline__ float2 vbt_w_deep(const SolveParams &P, int64_t traj, double t,
+                                                 int col) {
+  const uint32_t tj = uint32_t(traj);
+  const float2 z0 = vbt_normal_pair(P.seed, tj, 0u, kVbtRoot, col);
+  float ws0 = 0.f, ws1 = 0.f, wsu0 = z0.x, wsu1 = z0.y;
+  uint32_t node = 1;
+  // r 2^l, exact
+  float x = fminf(fmaxf(float((t - P.vbt_t0) * P.vbt_inv_len), 0.f), 1.f);
+#pragma unroll 1
+  for (int l = 0; l < P.vbt_deep; l++) {
+    const float2 z = vbt_normal_pair(P.seed, tj, node, kVbtMid, col);
+    const float a = __int_as_float((126 - ((l + 1) >> 1)) << 23) * (l & 1 ? 1.41421354f : 1.f);
+    // the half that holds r: its index among the level's is the largest integer below
+    // the scaled r, odd once that is a multiple of 2
+    x += x;
+    const bool right = x >= 16777216.f || (max(int(ceilf(x)) - 1, 0) & 1);
+    const float st0 = 0.5f * wsu0 + a * z.x, st1 = 0.5f * wsu1 + a * z.y;
+    if (right) {
+      ws0 += st0;
+      ws1 += st1;
+    }
+    wsu0 = right ? 0.5f * wsu0 - a * z.x : st0;
+    wsu1 = right ? 0.5f * wsu1 - a * z.y : st1;
+    node = 2 * node + (right ? 1u : 0u);
+  }
+  const float2 z = vbt_normal_pair(P.seed, tj, node, kVbtLeaf, col);
+  const float f = x < 16777216.f ? x - fmaxf(ceilf(x) - 1.f, 0.f) : 1.f;
+  const float su = P.vbt_deep < 127 ? __int_as_float((127 - P.vbt_deep) << 23) : 0.f;
+  const float bb = sqrtf(f * (1.f - f) * su), sq = P.vbt_sqrt_len;
+  return make_float2(sq * (ws0 + f * wsu0 + bb * z.x), sq * (ws1 + f * wsu1 + bb * z.y));
+}
+
 // Dimensions (col, col + 1).
 static __device__ __noinline__ float2 vbt_w_pair(const SolveParams &P, int64_t traj, double t,
                                                  int col) {
+  if (P.vbt_deep) return vbt_w_deep(P, traj, t, col);
   float w[2];
   vbt_w<2>(P, traj, t, col >> 2, col & 2, nullptr, w);
   return make_float2(w[0], w[1]);
 }
 
 // A quad of dimensions 4 quad .. 4 quad + 3, from the cached path.
-static __device__ __noinline__ float4 vbt_w_quad(const SolveParams &P, int64_t traj, double t,
-                                                 int quad, VbtQuadCache &C) {
+static __device__ __noinline__ float4 vbt_w_quad_word(const SolveParams &P, int64_t traj,
+                                                      double t, int quad, VbtQuadCache &C) {
   float w[4];
   vbt_w<4>(P, traj, t, quad, 0, &C, w);
   return make_float4(w[0], w[1], w[2], w[3]);
+}
+__device__ __forceinline__ float4 vbt_w_quad(const SolveParams &P, int64_t traj, double t,
+                                             int quad, VbtQuadCache &C) {
+  if (P.vbt_deep) {
+    const float2 a = vbt_w_deep(P, traj, t, 4 * quad), b = vbt_w_deep(P, traj, t, 4 * quad + 2);
+    return make_float4(a.x, a.y, b.x, b.y);
+  }
+  return vbt_w_quad_word(P, traj, t, quad, C);
 }
 
 // The tree with space-time Levy area: W_unit(r) and bar H_unit(r) = r H_{0,r}
