@@ -454,20 +454,6 @@ struct BsField {
 // share of sum (err / (atol + rtol max(|a0|, |a1|)))^2.  Otherwise da is added
 // to the CTA partial (Kahan).
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void kahan4(float *sum, float *comp, const float (&x)[4]) {
-  float4 s = *reinterpret_cast<float4 *>(sum), c = *reinterpret_cast<float4 *>(comp);
-  float sv[4] = {s.x, s.y, s.z, s.w}, cv[4] = {c.x, c.y, c.z, c.w};
-#pragma unroll
-  for (int q = 0; q < 4; q++) {
-    const float y = x[q] - cv[q];
-    const float t = sv[q] + y;
-    cv[q] = (t - sv[q]) - y;
-    sv[q] = t;
-  }
-  *reinterpret_cast<float4 *>(sum) = make_float4(sv[0], sv[1], sv[2], sv[3]);
-  *reinterpret_cast<float4 *>(comp) = make_float4(cv[0], cv[1], cv[2], cv[3]);
-}
-
 // (err / (atol + rtol max(|a0|, |a1|)))^2.  pid.py:475-492 scales a NaN
 // candidate by a0: fmaxf returns its non-NaN operand.  A NaN error
 // (infinite in _integrate.py:386) makes the row's norm NaN, which the
@@ -1154,30 +1140,6 @@ __device__ void bs_row_control(BsRows<M> &R, int r, float n_norm, const SolvePar
 // ---------------------------------------------------------------------------
 // The kernel.
 // ---------------------------------------------------------------------------
-// Yi = Y0 + sum_{j < i} a_ij K_j, the input of stage i.
-template <int SOLVER, int I, int S, int NE>
-__device__ __forceinline__ void stage_input(int i, const float (&Y0)[NE],
-                                            const float (&K)[S][NE], float (&Yi)[NE]) {
-  using TB = Tab<SOLVER>;
-  if constexpr (I < S) {
-    if (i == I) {
-#pragma unroll
-      for (int e = 0; e < NE; e++) {
-        float a = Y0[e];
-#pragma unroll
-        for (int j = 0; j < I; j++)
-          if (TB::a(I, j) != 0.0) a = fmaf(float(TB::a(I, j)), K[j][e], a);
-        Yi[e] = a;
-      }
-    } else {
-      stage_input<SOLVER, I + 1>(i, Y0, K, Yi);
-    }
-  } else {  // stage 0
-#pragma unroll
-    for (int e = 0; e < NE; e++) Yi[e] = Y0[e];
-  }
-}
-
 template <int SOLVER, int D, int H, bool PRECISE>
 __global__ void __launch_bounds__(256, 1) mlp_backsolve_kernel(SolveParams P, BsParams Q) {
   using SH = BsShape<D, H>;

@@ -806,6 +806,30 @@ __device__ void row_events(RowState<M> &R, RowEvents<M> &E, const RowEventStep<M
   }
 }
 
+// Yi = Y0 + sum_{j < i} a_ij K_j, the input of stage i.
+template <int SOLVER, int I, int S, int NE>
+__device__ __forceinline__ void stage_input(int i, const float (&Y0)[NE],
+                                            const float (&K)[S][NE], float (&Yi)[NE]) {
+  using TB = Tab<SOLVER>;
+  if constexpr (I < S) {
+    if (i == I) {
+#pragma unroll
+      for (int e = 0; e < NE; e++) {
+        float a = Y0[e];
+#pragma unroll
+        for (int j = 0; j < I; j++)
+          if (TB::a(I, j) != 0.0) a = fmaf(float(TB::a(I, j)), K[j][e], a);
+        Yi[e] = a;
+      }
+    } else {
+      stage_input<SOLVER, I + 1>(i, Y0, K, Yi);
+    }
+  } else {  // stage 0
+#pragma unroll
+    for (int e = 0; e < NE; e++) Yi[e] = Y0[e];
+  }
+}
+
 // ---------------------------------------------------------------------------
 // The kernel.
 // ---------------------------------------------------------------------------

@@ -432,30 +432,6 @@ __device__ __forceinline__ void fm_rows(const T *a, int row0, T (&v)[NE]) {
     *reinterpret_cast<int4 *>(v + e) = *reinterpret_cast<const int4 *>(a + row0 + e);
 }
 
-// Yi = Y0 + sum_{j < i} a_ij K_j, the input of stage i.
-template <int SOLVER, int I, int S, int NE>
-__device__ __forceinline__ void fm_stage_input(int i, const float (&Y0)[NE],
-                                               const float (&K)[S][NE], float (&Yi)[NE]) {
-  using TB = Tab<SOLVER>;
-  if constexpr (I < S) {
-    if (i == I) {
-#pragma unroll
-      for (int e = 0; e < NE; e++) {
-        float a = Y0[e];
-#pragma unroll
-        for (int j = 0; j < I; j++)
-          if (TB::a(I, j) != 0.0) a = fmaf(float(TB::a(I, j)), K[j][e], a);
-        Yi[e] = a;
-      }
-    } else {
-      fm_stage_input<SOLVER, I + 1>(i, Y0, K, Yi);
-    }
-  } else {  // stage 0
-#pragma unroll
-    for (int e = 0; e < NE; e++) Yi[e] = Y0[e];
-  }
-}
-
 // XO (extended outputs: SaveAt(steps=n), SaveAt(dense=True), the clip controller,
 // events, resume records) is a template flag, as in the trajectory kernels.
 template <int SOLVER, int D, int H, bool XO>
@@ -593,7 +569,7 @@ __global__ void __launch_bounds__((FmShape<D, H>::THREADS), 1) mlp_fm_kernel(Sol
     for (int e = 0; e < NE; e++) F[e] = F0[e];
 #pragma unroll 1
     for (int i = 0; i < S; i++) {
-      fm_stage_input<SOLVER, 1>(i, Y0, K, Yi);
+      stage_input<SOLVER, 1>(i, Y0, K, Yi);
       if (i > 0 || !TB::FSAL || any_first) {
         eval.put(Yi);
         eval(F);

@@ -768,7 +768,7 @@ __global__ void __launch_bounds__((FbShape<D, H, SDE>::THREADS), 1)
       float Yi[NE];
 #pragma unroll 1
       for (int i = 0; i < nf; i++) {
-        fm_stage_input<SOLVER, 1>(i, Y, K, Yi);
+        stage_input<SOLVER, 1>(i, Y, K, Yi);
         field.forward(Yi, F, sig, true);
 #pragma unroll
         for (int j = 0; j < S; j++)
@@ -782,7 +782,7 @@ __global__ void __launch_bounds__((FbShape<D, H, SDE>::THREADS), 1)
       if (anyfwd) {
         // ---- D. FWD rows: store the recomputed state -----------------------
         if constexpr (TB::SSAL) {
-          fm_stage_input<SOLVER, 1>(S - 1, Y, K, Y1);
+          stage_input<SOLVER, 1>(S - 1, Y, K, Y1);
         } else {
 #pragma unroll
           for (int e = 0; e < NE; e++) {
@@ -815,7 +815,7 @@ __global__ void __launch_bounds__((FbShape<D, H, SDE>::THREADS), 1)
                 Gs[e] = SDE ? KB[j][e] * dW[e] : 0.f;
               }
             }
-          fm_stage_input<SOLVER, 1>(i, Y, K, Yi);
+          stage_input<SOLVER, 1>(i, Y, K, Yi);
           field.forward(Yi, F, sig, false);  // x, a1, a2 (and sigma)
           field.backward(G, Gs, sig, gY);
         } else {
