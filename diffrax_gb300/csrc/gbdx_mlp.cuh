@@ -539,7 +539,7 @@ __device__ void row_control(RowState<M> &R, int r, int D, const SolveParams &P) 
 // the work by row -- the even lane descends the tree for r0, the odd lane for
 // r0 + 8, each for all four dimensions of the quad from its cached path -- and
 // swap halves.  Every lane of the warp must call it.
-template <class SH, class ROWS, int NE>
+template <class SH, bool DEEP, class ROWS, int NE>
 __device__ __forceinline__ void vbt_owned(const SolveParams &P, const ROWS &R, const int *flag,
                                           const double *tsel, VbtQuadCache &vc, float (&W)[NE],
                                           int warp, int lane) {
@@ -549,7 +549,7 @@ __device__ __forceinline__ void vbt_owned(const SolveParams &P, const ROWS &R, c
   const bool odd = lane & 1;
   const int myrow = odd ? row0 + 8 : row0;
   float4 w = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (flag[myrow]) w = vbt_w_quad(P, R.idx[myrow], tsel[myrow] * R.dir[myrow], col0 >> 2, vc);
+  if (flag[myrow]) w = vbt_w_quad<DEEP>(P, R.idx[myrow], tsel[myrow] * R.dir[myrow], col0 >> 2, vc);
   const float sx = odd ? w.x : w.z, sy = odd ? w.y : w.w;
   const float rx = __shfl_xor_sync(0xffffffffu, sx, 1), ry = __shfl_xor_sync(0xffffffffu, sy, 1);
   if (odd) {
@@ -566,12 +566,12 @@ __device__ __forceinline__ void vbt_owned(const SolveParams &P, const ROWS &R, c
 }
 
 // W(t0) of freshly loaded rows (SDE).
-template <class SH, int M, int NE>
+template <class SH, bool DEEP, int M, int NE>
 __device__ __forceinline__ void load_brownian(const SolveParams &P, const RowState<M> &R,
                                               VbtQuadCache &vc, float (&Wb)[NE], int warp,
                                               int lane) {
   float W[NE];
-  vbt_owned<SH>(P, R, R.loaded, R.tprev, vc, W, warp, lane);
+  vbt_owned<SH, DEEP>(P, R, R.loaded, R.tprev, vc, W, warp, lane);
 #pragma unroll
   for (int e = 0; e < NE; e++) {
     int row, col;
@@ -842,7 +842,8 @@ constexpr size_t mlp_events_offset() {
 // XO (extended outputs: SaveAt(steps=n), SaveAt(dense=True), the clip
 // controller and events) is a template flag, as in the trajectory kernels, so
 // that the kernels without them keep their registers.
-template <int SOLVER, int D, int H, bool PRECISE, bool SDE, bool XO>
+// DEEP (SDEs): the Brownian tree has more levels than a node number holds.
+template <int SOLVER, int D, int H, bool PRECISE, bool SDE, bool XO, bool DEEP = false>
 __global__ void __launch_bounds__(256) mlp_fused_kernel(SolveParams P) {
   using SH = MlpShape<D, H>;
   using FLD = MlpField<SH, PRECISE, SDE>;
@@ -895,7 +896,7 @@ __global__ void __launch_bounds__(256) mlp_fused_kernel(SolveParams P) {
   if constexpr (XO && TB::FSAL) {
     if (P.state_in) load_fsal_state<SH>(F0, P, R, warp, lane);
   }
-  if constexpr (SDE) load_brownian<SH>(P, R, vc, Wb, warp, lane);
+  if constexpr (SDE) load_brownian<SH, DEEP>(P, R, vc, Wb, warp, lane);
   __syncthreads();
   if (tid < M) R.loaded[tid] = 0;
 
@@ -923,7 +924,7 @@ __global__ void __launch_bounds__(256) mlp_fused_kernel(SolveParams P) {
     if constexpr (SDE) {
       // Brownian increment over [tprev, tnext] of every owned element; W at
       // tprev is carried from the previous accepted step.
-      vbt_owned<SH>(P, R, R.live, R.tnext, vc, Wn, warp, lane);
+      vbt_owned<SH, DEEP>(P, R, R.live, R.tnext, vc, Wn, warp, lane);
 #pragma unroll
       for (int e = 0; e < NE; e++) dW[e] = Wn[e] - Wb[e];
     }
@@ -1317,7 +1318,7 @@ __global__ void __launch_bounds__(256) mlp_fused_kernel(SolveParams P) {
       if constexpr (XO && TB::FSAL) {
         if (P.state_in) load_fsal_state<SH>(F0, P, R, warp, lane);
       }
-      if constexpr (SDE) load_brownian<SH>(P, R, vc, Wb, warp, lane);
+      if constexpr (SDE) load_brownian<SH, DEEP>(P, R, vc, Wb, warp, lane);
       __syncthreads();
       if (tid < M) R.loaded[tid] = 0;
     }

@@ -220,7 +220,7 @@ __device__ void bwd_row_init(BwdRows<SH::M> &R, int r, int64_t i, const SolvePar
   }
 }
 
-template <int SOLVER, int D, int H, bool SDE>
+template <int SOLVER, int D, int H, bool SDE, bool DEEP = false>
 __global__ void __launch_bounds__(256) mlp_bwd_kernel(SolveParams P, BwdParams Q) {
   using SH = MlpShape<D, H>;
   using FLD = MlpField<SH, true, SDE>;
@@ -345,8 +345,8 @@ __global__ void __launch_bounds__(256) mlp_bwd_kernel(SolveParams P, BwdParams Q
       // the lane's cached tree path (consecutive evaluations lie within a
       // step or two).
       float wa[NE], wb[NE];
-      vbt_owned<SH>(P, R, R.w_lo, R.t_lo, vc, wa, warp, lane);
-      vbt_owned<SH>(P, R, R.w_hi, R.t_hi, vc, wb, warp, lane);
+      vbt_owned<SH, DEEP>(P, R, R.w_lo, R.t_lo, vc, wa, warp, lane);
+      vbt_owned<SH, DEEP>(P, R, R.w_hi, R.t_hi, vc, wb, warp, lane);
 #pragma unroll
       for (int e = 0; e < NE; e++) {
         int row, col;

@@ -11,6 +11,8 @@ template <int SOLVER, int D, int H, bool SDE>
 cudaError_t launch_mlp_bwd(const SolveParams &P, const BwdParams &Q, int grid, cudaStream_t s) {
   using Sm = typename MlpVjp<MlpShape<D, H>, SDE>::Sm;
   auto k = mlp_bwd_kernel<SOLVER, D, H, SDE>;
+  if constexpr (SDE)
+    if (P.vbt_deep) k = mlp_bwd_kernel<SOLVER, D, H, SDE, true>;
   cudaError_t e =
       cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Sm));
   if (e != cudaSuccess) return e;

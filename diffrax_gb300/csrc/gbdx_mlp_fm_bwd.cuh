@@ -290,7 +290,7 @@ __device__ __forceinline__ void fb_spread(int i, const float (&g)[NE], float (&K
 // Brownian values at times tsel[row] of the owned elements of the rows with flag
 // set.  The four lanes of a quad of dimensions each descend the tree for one of
 // the four owned rows, for all four dimensions, and exchange.
-template <class SH>
+template <class SH, bool DEEP>
 __device__ __forceinline__ void fb_brownian(const SolveParams &P, const BwdRows<SH::R> &R,
                                             const int *flag, const double *tsel,
                                             VbtQuadCache &vc, float (&W)[SH::NE],
@@ -298,7 +298,7 @@ __device__ __forceinline__ void fb_brownian(const SolveParams &P, const BwdRows<
   static_assert(SH::NE == 4, "a quad's lanes take one row each");
   const int me = m.tl & 3, row = m.row0 + me;
   float4 w = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (flag[row]) w = vbt_w_quad(P, R.idx[row], tsel[row] * R.dir[row], m.f >> 2, vc);
+  if (flag[row]) w = vbt_w_quad<DEEP>(P, R.idx[row], tsel[row] * R.dir[row], m.f >> 2, vc);
   // round x: dimension me ^ x of my row goes to lane me ^ x, whose row's value
   // of my dimension comes back
 #pragma unroll
@@ -530,7 +530,7 @@ __device__ __forceinline__ void fb_flush(uint32_t lanes, int tcol, float *psum, 
   }
 }
 
-template <int SOLVER, int D, int H, bool SDE>
+template <int SOLVER, int D, int H, bool SDE, bool DEEP = false>
 __global__ void __launch_bounds__((FbShape<D, H, SDE>::THREADS), 1)
     mlp_fm_bwd_kernel(SolveParams P, BwdParams Q) {
   using SH = FbShape<D, H, SDE>;
@@ -689,8 +689,8 @@ __global__ void __launch_bounds__((FbShape<D, H, SDE>::THREADS), 1)
         // W at both ends of the step; a row's consecutive iterations share an end,
         // whose value its threads carry (gbdx_mlp_bwd.cuh)
         float wa[NE], wb[NE];
-        fb_brownian<SH>(P, R, R.w_lo, R.t_lo, vc, wa, m);
-        fb_brownian<SH>(P, R, R.w_hi, R.t_hi, vc, wb, m);
+        fb_brownian<SH, DEEP>(P, R, R.w_lo, R.t_lo, vc, wa, m);
+        fb_brownian<SH, DEEP>(P, R, R.w_hi, R.t_hi, vc, wb, m);
 #pragma unroll
         for (int e = 0; e < NE; e++) {
           const int row = m.row0 + e;
@@ -949,6 +949,8 @@ cudaError_t launch_fm_bwd(const SolveParams &P, const BwdParams &Q, int grid, cu
   constexpr size_t bytes = sizeof(FbSmem<SH>);
   static_assert(bytes <= 227 * 1024 && bytes > 114 * 1024, "one CTA per SM");
   auto k = mlp_fm_bwd_kernel<SOLVER, D, H, SDE>;
+  if constexpr (SDE)
+    if (P.vbt_deep) k = mlp_fm_bwd_kernel<SOLVER, D, H, SDE, true>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   if (e != cudaSuccess) return e;
   if (P.batch <= 0) return cudaSuccess;

@@ -23,6 +23,8 @@ cudaError_t launch_mlp(const SolveParams &P, const LaunchCfg &cfg, cudaStream_t 
   constexpr size_t bytes = mlp_smem_bytes<D, H, PRECISE, SDE, XO>();
   static_assert(bytes <= 227 * 1024, "shared memory of one CTA");
   auto k = mlp_fused_kernel<SOLVER, D, H, PRECISE, SDE, XO>;
+  if constexpr (SDE)
+    if (P.vbt_deep) k = mlp_fused_kernel<SOLVER, D, H, PRECISE, SDE, XO, true>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   if (e != cudaSuccess) return e;
   if (P.batch <= 0) return cudaSuccess;

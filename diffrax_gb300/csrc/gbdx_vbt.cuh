@@ -250,10 +250,7 @@ __device__ __forceinline__ void vbt_w(const SolveParams &P, int64_t traj, double
 
 // The same for dimensions (col, col + 1) of a deeper tree, level by level: each takes the
 // turn that r scaled to it says, and the node's number is kept modulo 2^32, as the draws
-// take it.  (A function of its own, one pair and one level at a time: its registers count
-// for every kernel that may call it, and 80 are what lets three CTAs of the neural SDE
-// share an SM; with turns of both kinds in vbt_w 32768 trajectories took 3.40 instead of
-// 3.33 ms, with a copy of vbt_w for quads 3.9.)
+// take it.
 static __device__ __noinline__ float2 vbt_w_deep(const SolveParams &P, int64_t traj, double t,
                                                  int col) {
   const uint32_t tj = uint32_t(traj);
@@ -296,19 +293,24 @@ static __device__ __noinline__ float2 vbt_w_pair(const SolveParams &P, int64_t t
 }
 
 // A quad of dimensions 4 quad .. 4 quad + 3, from the cached path.
-static __device__ __noinline__ float4 vbt_w_quad_word(const SolveParams &P, int64_t traj,
-                                                      double t, int quad, VbtQuadCache &C) {
+static __device__ __noinline__ float4 vbt_w_quad(const SolveParams &P, int64_t traj, double t,
+                                                 int quad, VbtQuadCache &C) {
   float w[4];
   vbt_w<4>(P, traj, t, quad, 0, &C, w);
   return make_float4(w[0], w[1], w[2], w[3]);
 }
+
+// The same of a tree of either depth class; the launch chooses the kernel by vbt_deep.
+// (A choice in the kernel cost 4000 neural SDE trajectories 3 %, 955 to 988 us.)
+template <bool DEEP>
 __device__ __forceinline__ float4 vbt_w_quad(const SolveParams &P, int64_t traj, double t,
                                              int quad, VbtQuadCache &C) {
-  if (P.vbt_deep) {
+  if constexpr (DEEP) {
     const float2 a = vbt_w_deep(P, traj, t, 4 * quad), b = vbt_w_deep(P, traj, t, 4 * quad + 2);
     return make_float4(a.x, a.y, b.x, b.y);
+  } else {
+    return vbt_w_quad(P, traj, t, quad, C);
   }
-  return vbt_w_quad_word(P, traj, t, quad, C);
 }
 
 // The tree with space-time Levy area: W_unit(r) and bar H_unit(r) = r H_{0,r}

@@ -88,3 +88,39 @@ def test_below_the_smallest_float(tol):
     got = solve(ou(tol, 2), False, y0, args)[0].ys
     want = solve(ou(2.0 ** -28, 2), False, y0, args)[0].ys
     assert float((got - want).abs().max()) < 2e-5 * float(want.abs().max())
+
+
+def neural(tol, precision, grad):
+    """A neural SDE on the path of a tree of tolerance tol, at exact times."""
+    dev, w = torch.device("cuda"), (32, 64, 64, 32)
+    gen = torch.Generator(device=dev).manual_seed(9)
+    leaf = lambda *s: torch.randn(*s, device=dev, generator=gen).div_(  # noqa: E731
+        s[-1] ** 0.5).requires_grad_(grad)
+    Ws, bs = [leaf(w[i + 1], w[i]) for i in range(3)], [leaf(w[i + 1]) for i in range(3)]
+    Wd, bd, y0 = leaf(32, 32), leaf(32), leaf(45, 32)
+    terms = dfx.MultiTerm(dfx.ODETerm(dfx.MLPField(Ws, bs, precision=precision)), dfx.ControlTerm(
+        dfx.TanhDiagonalDiffusion(Wd, bd), dfx.VirtualBrownianTree(0.0, 1.0, tol, (32,), key=3)))
+    return terms, y0, [y0, *Ws, *bs, Wd, bd]
+
+
+@pytest.mark.parametrize("precision", ["bf16", "fp32"])
+@pytest.mark.parametrize("tol", [2.0 ** -31, 1e-10, 1e-60])
+def test_gradients(tol, precision):
+    # the path at the steps' times is that of a tree that resolves them (2e-5, above)
+    grads = []
+    for t in (tol, 2.0 ** -28):
+        terms, y0, leaves = neural(t, precision, True)
+        sol = dfx.diffeqsolve(terms, dfx.Heun(), 0.0, N * H, H, y0)
+        grads.append(torch.autograd.grad(sol.ys.square().sum(), leaves))
+    for a, b in zip(*grads):
+        assert float((a - b).norm()) <= 2e-5 * float(b.norm())
+
+
+@pytest.mark.parametrize("precision", ["bf16", "fp32"])
+def test_extended_outputs(precision):
+    ys = []
+    for t in (1e-10, 2.0 ** -28):
+        terms, y0, _ = neural(t, precision, False)
+        ys.append(dfx.diffeqsolve(terms, dfx.Heun(), 0.0, N * H, H, y0, max_steps=N,
+                                  saveat=dfx.SaveAt(steps=True)).ys)
+    assert float((ys[0] - ys[1]).abs().max()) <= 2e-5 * float(ys[1].abs().max())
