@@ -717,7 +717,7 @@ class _NeuralCase:
             self.widths, self.B, seed = [32, 64, 64, 32], 32768, 23
             self.solver, self.ctrl, self.dt0 = dfx.Heun(), dfx.ConstantStepSize(), 0.01
             self.ts, self.sde = None, True
-            # the default checkpoint count (ceil(log2(max_steps)))
+            # the default checkpoint count
             self.adjoint = dfx.RecursiveCheckpointAdjoint()
             self.name = "neural_sde_32_64_heun_dt0.01_vbt1e-3_b32768_recursive"
         self.saveat = dfx.SaveAt(ts=self.ts) if self.ts is not None else dfx.SaveAt(t1=True)

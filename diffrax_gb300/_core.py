@@ -62,7 +62,10 @@ class MLPField(AbstractField):
     accumulation: the weights are held as BF16 values and every activation
     operand is split into three BF16 pieces (24 significant bits, three
     products per tile), so the field equals an FP32 evaluation of the
-    BF16-rounded weights and stays smooth under adaptive stepping.  "fp32"
+    BF16-rounded weights and stays smooth under adaptive stepping.  (ODE
+    solves for a recursive gradient run another kernel than the rest: equal to
+    FP32 rounding on a constant grid, but under an adaptive controller its
+    steps, and so the last digits within the tolerance, differ.)  "fp32"
     runs the products in FP32 on the CUDA cores with the FP32 weights (parity
     mode)."""
     field_id = 3

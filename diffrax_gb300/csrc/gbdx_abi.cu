@@ -605,9 +605,11 @@ int gbdx_problem_create(const gbdx_problem_desc *desc, gbdx_problem **out) {
     if (!precise && !sde) {
       // BF16 ODEs: the feature-major tcgen05 form, except where a recursive adjoint
       // records its tape.  The row-tile form's noisier products make its embedded error
-      // estimate larger (5.36 against 5.03 accepted steps on the 64-128-128-64 field),
-      // and its smaller steps keep dL/dy0 within 1.7e-6 of the continuous solution's,
-      // against 1.9e-6; on equal grids the feature-major form is the more exact one.
+      // estimate larger (rtol 1e-5, 64-128-128-64: 5.36 against 5.03 accepted steps), and
+      // its smaller steps kept dL/dy0 within 1.7e-6 of the continuous solution's, against
+      // 1.9e-6; at 32-64-64-32 it takes 5.17 against 5.04 steps and ends 4.9e-7 from the
+      // solution, against 5.8e-7.  On equal grids the feature-major form is the more exact
+      // one.
       const bool tape = d.adjoint == GBDX_ADJ_RECURSIVE;
       if (D == 64 && H == 128) {
         p->ode_xo = gbdx::find_mlp_fm_xo_entry_d64h128(d.solver);

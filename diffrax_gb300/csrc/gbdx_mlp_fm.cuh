@@ -30,9 +30,13 @@
 // of 16 rows and 4 warps measured 8700 cycles a stage of 64 rows at width 128
 // against 6400 with two of 32 rows and 8 warps.
 //
-// Bound: the epilogues' issue slots (~27 a warp and element: tanh, splitting and
-// storing, sums), about 3500 cycles of a stage of 64 rows at width 128, then the chain
-// of barriers and product latencies.  Measured (Tsit5 PID(1e-5, 1e-7) on [0, 1], kernel
+// Bound: the serial chain of a stage (three products, the waits for their completion and
+// the reads of their sums, barriers of eight warps), which two groups overlap in part, and
+// in it the epilogues' issue slots (~27 a warp and element: tanh, splitting and storing,
+// sums; about 3500 of a stage's 6400 cycles with 64 rows at width 128).  Counters at 8192
+// rows: issue slots 37 % (61 % on the fullest SM), tensor pipe 19 %, of 10.8 warp cycles an
+// issue 2.4 on those reads and 2.3 on barriers; width 256, 16384 rows: 40 (59), 28 %, 2.7
+// of 9.9 and 0.8.  Measured (Tsit5 PID(1e-5, 1e-7) on [0, 1], kernel
 // time) against the mma.sync row tiles that it replaced: 64-128-128-64 at 8192 rows
 // 421 -> 210 us, at 19456 902 -> 371 us (445 us with 128 trajectories on the lanes);
 // 64-256-256-64 with 32 saves at 16384 rows 2240 -> 780 us.

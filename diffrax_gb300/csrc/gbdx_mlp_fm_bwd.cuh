@@ -28,7 +28,8 @@
 // the accumulators' lanes are full in both directions (gbdx_mlp_fm.cuh: lane maps).
 //
 // Bound: the serial chain of a stage (six products, their completion latency and
-// epilogues); one tile a CTA.
+// epilogues), one tile a CTA: at 64-128 and 8192 rows issue slots 27 %, tensor pipe 18 %; the
+// neural SDE 24 and 11 %.
 #pragma once
 
 #include "gbdx_mlp_bwd.cuh"
